@@ -34,7 +34,7 @@ template <> __device__ __forceinline__ const Tables<9> &tab<9>() { return c_tab9
 // fully inlined sweep outgrew the instruction cache (ncu: instruction-fetch stalls of 2.5
 // cycles per issued instruction, the largest stall); out of line, the FP64 step took
 // 7.38 ms instead of 9.73 ms at 256x256x128. The arithmetic is the same either way.
-static __device__ __noinline__ double pow_gamma_call(double x) { return pow_cr(x, GAMMA); }
+static __device__ __noinline__ double pow_gamma_call(double x) { return pow_gamma_cr(x); }
 __device__ __forceinline__ double pow_gamma(double x) { return pow_gamma_call(x); }
 template <class Sc> __device__ __forceinline__ Sc pow_gamma(const Sc &x) { return pow_cr(x, GAMMA); }
 

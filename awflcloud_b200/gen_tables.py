@@ -42,6 +42,8 @@ import mpmath as mp
 
 mp.mp.prec = 256
 HALF = mp.mpf(1) / 2
+GAMMA = 1.40027894002789400278940027894  # cp/cv, rounded to the double the path uses
+POWG_E0, POWG_NE = 4, 6  # binary exponents of rho*theta with a table of their own: [16, 1024)
 
 
 # ----------------------------------------------------------------------------- rounding
@@ -322,7 +324,10 @@ def emit_pow_header() -> str:
     """Tables of the correctly rounded pow (csrc/awfl_pow.cuh):
     log: for j in 0..127, inv_j = double(1 / (1 + (j + 1/2)/128)) and -ln(inv_j) as a
     double-double; exp: 2^(j/64) for j in 0..63 as double-doubles; ln2 split as
-    L2HI (42 bits) + L2LO, and ln2/64 split as E1 (36 bits) + E2."""
+    L2HI (42 bits) + L2LO, and ln2/64 split as E1 (36 bits) + E2. For the pressure's own
+    exponent gamma (the double): (2^e/inv_j)^gamma for e in POWG_E0..POWG_E0+POWG_NE-1 and
+    every j as double-doubles (hi, lo interleaved, index (e - POWG_E0)*128 + j), and the
+    binomial coefficients C(gamma, n), n = 2 as a double-double, 3..7."""
     out = ["// GENERATED by awflcloud_b200/gen_tables.py -- do not edit by hand.\n",
            "// Tables for awfl_pow.cuh (values exact to 256 bits before rounding).\n",
            "#pragma once\n\n",
@@ -361,6 +366,23 @@ def emit_pow_header() -> str:
     out.append("#define AWFL_POW_L2HI %s\n#define AWFL_POW_L2LO %s\n" % (hexlit(l2hi), hexlit(l2lo)))
     out.append("#define AWFL_POW_E1 %s\n#define AWFL_POW_E2 %s\n#define AWFL_POW_INV_E %s\n"
                % (hexlit(e1), hexlit(e2), hexlit(inv64)))
+    g = mp.mpf(GAMMA)
+    tab = []
+    for e in range(POWG_E0, POWG_E0 + POWG_NE):
+        for j in range(128):
+            v = (mp.mpf(2) ** e / mp.mpf(inv[j])) ** g
+            hi = float(_round_mant(v, 53))
+            tab += [hi, float(_round_mant(v - mp.mpf(hi), 53))]
+    out.append("#define AWFL_POWG_E0 %d\n#define AWFL_POWG_NE %d\n" % (POWG_E0, POWG_NE))
+    out.append("#ifdef __CUDACC__\n__device__ __align__(16) const double\n#else\nstatic const double\n#endif\n")
+    out.append("awfl_powg_tab[%d] = {%s};\n" % (len(tab), ", ".join(hexlit(v) for v in tab)))
+    c = g
+    for n in range(2, 8):
+        c = c * (g - (n - 1)) / n
+        hi = float(_round_mant(c, 53))
+        out.append("#define AWFL_POWG_C%d %s\n" % (n, hexlit(hi)))
+        if n == 2:
+            out.append("#define AWFL_POWG_C2L %s\n" % hexlit(float(_round_mant(c - mp.mpf(hi), 53))))
     return "".join(out)
 
 
