@@ -18,6 +18,7 @@
 #include "awfl_adj_split.h"
 #include "awfl_internal.h"
 #include "awfl_netcdf.h"
+#include "awfl_recip.h"
 #include "awfl_tables.h"
 
 using namespace awfl;
@@ -233,8 +234,8 @@ int ensure_tables(awfl_ctx *c) {
     std::memcpy(t.deriv, c->deriv.data(), sizeof t.deriv);
     std::memcpy(t.idl, c->idl.data(), sizeof t.idl);
     t.sigma = c->sigma;
-    t.ridl = 1.0 / t.idl[t.HS + 1];
     std::memcpy(t.wts, c->wts_ngll.data(), sizeof t.wts);
+    if (!host::complete_tables(t)) return fail(c, AWFL_ERR_STATE, "transform tables without the expected structure");
     e = upload_tables_fp64(5, &t, sizeof t);
     if (e == cudaSuccess) e = upload_tables_adj(5, &t, sizeof t);
     if (e == cudaSuccess) e = upload_tables_tracers(5, &t, sizeof t);
@@ -248,8 +249,8 @@ int ensure_tables(awfl_ctx *c) {
     std::memcpy(t.deriv, c->deriv.data(), sizeof t.deriv);
     std::memcpy(t.idl, c->idl.data(), sizeof t.idl);
     t.sigma = c->sigma;
-    t.ridl = 1.0 / t.idl[t.HS + 1];
     std::memcpy(t.wts, c->wts_ngll.data(), sizeof t.wts);
+    if (!host::complete_tables(t)) return fail(c, AWFL_ERR_STATE, "transform tables without the expected structure");
     e = upload_tables_fp64(9, &t, sizeof t);
     if (e == cudaSuccess) e = upload_tables_adj(9, &t, sizeof t);
     if (e == cudaSuccess) e = upload_tables_tracers(9, &t, sizeof t);

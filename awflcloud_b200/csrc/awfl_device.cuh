@@ -144,12 +144,156 @@ __device__ __forceinline__ void reconstruct_gll(const Sc (&sten)[ORD], Sc (&out)
   }
 }
 
+// The WENO reconstruction on doubles with the general routine's results (weno_coefs and the
+// GLL evaluation above) in about half of its FP64 instructions; the FP64 pipe bounds the
+// sweep. What is left out changes no bit:
+//   - products with structural zeros, and sums that start at 0 +: the sign of a zero is all
+//     they can change, and the last sum of each GLL value, which does start at +0, drops it;
+//   - a product by a power of two is exact, so it goes with its sum into one FMA;
+//   - ord 5 shares products: u/24, u/12 and u/6 are one rounded product scaled by 2 and 4;
+//   - the weights' divisions by div_near, interleaved (no branch per division), the bridge
+//     polynomial's by div_known; the mapping's constants come from the tables.
+// A stencil whose smoothness indicators leave the range in which these hold (tv^2 >= 2^300,
+// infinities and NaN among them) is left to the general routine: these return false.
+// 256x256x128: ord 5 6.68 -> 4.86 ms per step; 128x128x64, ord 9: 3.99 -> 3.30 ms.
+template <int ORD>
+__device__ __forceinline__ bool weno_weights(const double (&tv)[(ORD + 3) / 2], double (&w)[(ORD + 3) / 2]) {
+  constexpr int HS = (ORD - 1) / 2;
+  const Tables<ORD> &T = tab<ORD>();
+  unsigned top = 0;
+#pragma unroll
+  for (int i = 0; i < HS + 2; i++) {
+    w[i] = tv[i] * tv[i] + 1.0e-20;
+    top = max(top, (unsigned)__double2hiint(w[i]));
+  }
+  if (top >= ((1023u + 300u) << 20)) return false;
+#pragma unroll
+  for (int i = 0; i < HS + 2; i++) w[i] = div_near(T.idl[i], w[i], rcp_near(w[i]));
+  auto convexify = [&]() {
+    double sum = w[0];
+#pragma unroll
+    for (int i = 1; i < HS + 2; i++) sum += w[i];
+    sum += 1.0e-20;
+    const double y = rcp_near(sum);
+#pragma unroll
+    for (int i = 0; i < HS + 2; i++) w[i] = div_near(w[i], sum, y);
+  };
+  convexify();
+#pragma unroll
+  for (int i = 0; i < HS + 2; i++) {
+    const double den = T.map_c[i] + w[i] * T.map_d[i];
+    w[i] = div_near(w[i] * (T.map_a[i] - T.map_b[i] * w[i] + w[i] * w[i]), den, rcp_near(den));
+  }
+  convexify();
+  return true;
+}
+// the high-order candidate's smoothness indicator relaxed towards the others' mean
+template <int HS> __device__ __forceinline__ void relax_tv(double (&tv)[HS + 2], double sigma) {
+  double avg = tv[0];
+#pragma unroll
+  for (int i = 1; i < HS + 1; i++) avg += tv[i];
+  avg = divk(avg, HS + 1);
+  tv[HS + 1] = avg + (tv[HS + 1] - avg) * sigma;
+}
+template <int ORD>
+__device__ __forceinline__ bool weno_gll(const double (&u)[ORD], double (&out)[OrdTraits<ORD>::NGLL]) {
+  constexpr int HS = (ORD - 1) / 2;
+  constexpr int NG = OrdTraits<ORD>::NGLL;
+  const Tables<ORD> &T = tab<ORD>();
+  double a[HS + 1][HS + 1], h[ORD];
+  if constexpr (ORD == 5) {
+    const double p0 = kW24 * u[0], p1 = kW24 * u[1], p3 = kW24 * u[3], p4 = kW24 * u[4];
+    const double l0 = __fma_rn(2., p1, -p0), c2 = kW2324 * u[2], t2 = 1.5 * u[2];
+    const double h0 = .5 * u[0], h1 = .5 * u[1], h2 = .5 * u[2];
+    a[0][0] = l0 + c2;
+    a[0][1] = __fma_rn(-2., u[1], h0) + t2;
+    a[0][2] = __fma_rn(.5, u[2], h0 - u[1]);
+    a[1][0] = (kW1312 * u[2] - p1) - p3;
+    a[1][1] = __fma_rn(.5, u[3], -h1);
+    a[1][2] = __fma_rn(.5, u[3], h1 - u[2]);
+    a[2][0] = __fma_rn(2., p3, c2) - p4;
+    a[2][1] = __fma_rn(-.5, u[4], __fma_rn(2., u[3], -t2));
+    a[2][2] = __fma_rn(.5, u[4], h2 - u[3]);
+    h[0] = (((kH00 * u[0] - kH10 * u[1]) + kH20 * u[2]) - kH10 * u[3]) + kH00 * u[4];
+    h[1] = ((kH01 * u[0] - kH11 * u[1]) + kH11 * u[3]) - kH01 * u[4];
+    h[2] = __fma_rn(-.0625, u[4], (__fma_rn(-.0625, u[0], .75 * u[1]) - 1.375 * u[2]) + .75 * u[3]);
+    h[3] = 2. * (__fma_rn(-2., p3, l0) + p4);
+    h[4] = __fma_rn(-4., p3, __fma_rn(.25, u[2], __fma_rn(-4., p1, p0))) + p4;
+  } else {
+#pragma unroll
+    for (int i = 0; i < HS + 1; i++)
+#pragma unroll
+      for (int ii = 0; ii < HS + 1; ii++) {
+        double acc = T.recon[i * ORD * ORD + ii] * u[i];
+#pragma unroll
+        for (int s = 1; s < HS + 1; s++) {
+          if (HS % 2 == 0 && i == HS / 2 && s == HS / 2 && ii % 2 == 1) continue;
+          acc += T.recon[(i * ORD + s) * ORD + ii] * u[i + s];
+        }
+        a[i][ii] = acc;
+      }
+#pragma unroll
+    for (int ii = 0; ii < ORD; ii++) {
+      double acc = T.recon[(HS + 1) * ORD * ORD + ii] * u[0];
+#pragma unroll
+      for (int s = 1; s < ORD; s++) {
+        if (s == HS && ii % 2 == 1) continue;
+        acc += T.recon[((HS + 1) * ORD + s) * ORD + ii] * u[s];
+      }
+      h[ii] = acc;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < HS + 1; i++)
+#pragma unroll
+    for (int ii = 0; ii < HS + 1; ii++) h[ii] -= T.idl[i] * a[i][ii];
+#pragma unroll
+  for (int ii = 0; ii < ORD; ii++) h[ii] = div_known(h[ii], T.ridl_h, T.ridl_l);
+  double tv[HS + 2], w[HS + 2];
+#pragma unroll
+  for (int i = 0; i < HS + 1; i++) tv[i] = tv_eval<HS + 1>(a[i]);
+  tv[HS + 1] = tv_eval<ORD>(h);
+  relax_tv<HS>(tv, T.sigma);
+  if (!weno_weights<ORD>(tv, w)) return false;
+#pragma unroll
+  for (int ii = 0; ii < ORD; ii++) {
+    if (ii <= HS) {
+      double acc = w[0] * a[0][ii];
+#pragma unroll
+      for (int i = 1; i < HS + 1; i++) acc += w[i] * a[i][ii];
+      h[ii] = acc + w[HS + 1] * h[ii];
+    } else {
+      h[ii] = w[HS + 1] * h[ii];
+    }
+  }
+  const double mid = h[0] + 0.;  // +0 for a zero of either sign, as a sum from +0 gives
+#pragma unroll
+  for (int ii = 0; ii < NG; ii++) {
+    double acc = mid;
+    if (ii != NG / 2) {
+#pragma unroll
+      for (int s = 1; s < ORD; s++) {
+        const double c = T.c2g[s * NG + ii];
+        if (ii == 0 || ii == NG - 1) acc = __fma_rn((s % 2 && ii == 0) ? -1. / (1 << s) : 1. / (1 << s), h[s], acc);
+        else acc += c * h[s];
+      }
+    }
+    out[ii] = acc;
+  }
+  return true;
+}
+
 template <int ORD> struct StenV { double v[ORD]; };
 template <int ORD> struct GllV { double v[OrdTraits<ORD>::NGLL]; };
-template <int ORD> static __device__ __noinline__ GllV<ORD> reconstruct_gll_call(StenV<ORD> s, bool doweno) {
+template <int ORD> static __device__ __noinline__ GllV<ORD> reconstruct_gll_general(StenV<ORD> s, bool doweno) {
   GllV<ORD> o;
   reconstruct_gll<ORD>(s.v, o.v, doweno);
   return o;
+}
+template <int ORD> static __device__ __noinline__ GllV<ORD> reconstruct_gll_call(StenV<ORD> s, bool doweno) {
+  GllV<ORD> o;
+  if (doweno && weno_gll<ORD>(s.v, o.v)) return o;
+  return reconstruct_gll_general<ORD>(s, doweno);
 }
 template <int ORD, class Sc>
 __device__ __forceinline__ void reconstruct_gll_any(const Sc (&sten)[ORD], Sc (&out)[OrdTraits<ORD>::NGLL],

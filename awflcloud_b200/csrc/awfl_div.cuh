@@ -21,6 +21,20 @@
 // carries IEEE's sign of zero. Tested against the GPU's IEEE division on random and
 // edge-case operands (tests/test_pow_gpu.py) and through the bit-exact parity tests.
 //
+// The reciprocal itself comes from Newton iterations on the GPU's reciprocal seed
+// (rcp.approx.ftz.f64, 20 bits), one cubic step and one with the residual b*y - 1 exact
+// (Markstein, ibid.): RN(1/b) for every significand but all ones, where y is the value on
+// the other side of the midpoint that 1/b all but is. No branch, unlike 1.0/b, so that the
+// divisions of independent points overlap. Shorter forms where they suffice:
+//   divp        divr without the test for a zero dividend: forming the remainder as
+//               b*q - a keeps a zero's sign through the corrections for b > 0
+//   div_known   a divisor known on the host, 1/b = h + l: two instructions (awfl_recip.h)
+//   div_near    one correction instead of two: q0 is within 1.5 ulp, and the corrected
+//               value before its rounding within 2^-104 of a/b, so that the quotient is
+//               the IEEE one unless a/b lies that close to a rounding midpoint (one pair of
+//               operands in ~2^50); for the WENO weights, whose divisions do not share a
+//               divisor
+//
 // The scalar type may also be the tangent-linear Dual; its quotients keep the plain
 // division (their value parts are bit-identical either way).
 #pragma once
@@ -34,8 +48,26 @@ template <> struct Rcp<double> {
   double b, y;  // divisor and RN(1/b)
 };
 
+__device__ __forceinline__ double rcp_seed(double b) {
+#ifdef __CUDA_ARCH__
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+  return y;
+#else  // a host build of this header: a seed of the same 20 bits
+  return __hiloint2double(__double2hiint(1.0 / b), 0);
+#endif
+}
+// 1/b within 2^-53 (1 + 2^-5) of itself
+__device__ __forceinline__ double rcp_near(double b) {
+  const double y = rcp_seed(b), e = __fma_rn(-b, y, 1.0);
+  return __fma_rn(__fma_rn(e, e, e), y, y);
+}
+
 template <class Sc> __device__ __forceinline__ Rcp<Sc> make_rcp(const Sc &b) { return Rcp<Sc>{b}; }
-template <> __device__ __forceinline__ Rcp<double> make_rcp(const double &b) { return Rcp<double>{b, 1.0 / b}; }
+template <> __device__ __forceinline__ Rcp<double> make_rcp(const double &b) {
+  const double y = rcp_near(b);
+  return Rcp<double>{b, __fma_rn(__fma_rn(-b, y, 1.0), y, y)};
+}
 // a divisor whose reciprocal RN(1/b) is already known (host-computed, or a folded constant)
 __host__ __device__ __forceinline__ Rcp<double> rcp_known(double b, double y) { return Rcp<double>{b, y}; }
 
@@ -44,6 +76,20 @@ __device__ __forceinline__ double div_markstein(double a, double b, double y) {
   const double q1 = __fma_rn(__fma_rn(-q0, b, a), y, q0);
   const double q2 = __fma_rn(__fma_rn(-q1, b, a), y, q1);
   return a == 0.0 ? q0 : q2;
+}
+
+__device__ __forceinline__ double div_near(double a, double b, double y) {
+  const double q = __dmul_rn(a, y);
+  return __fma_rn(__fma_rn(q, b, -a), -y, q);
+}
+__device__ __forceinline__ double div_known(double a, double h, double l) { return __fma_rn(a, h, __dmul_rn(a, l)); }
+
+// a / r.b, correctly rounded, for r.b > 0
+template <class Sc> __device__ __forceinline__ Sc divp(const Sc &a, const Rcp<Sc> &r) { return a / r.b; }
+__device__ __forceinline__ double divp(const double &a, const Rcp<double> &r) {
+  const double q0 = __dmul_rn(a, r.y);
+  const double q1 = __fma_rn(__fma_rn(q0, r.b, -a), -r.y, q0);
+  return __fma_rn(__fma_rn(q1, r.b, -a), -r.y, q1);
 }
 
 // a / r.b, correctly rounded
@@ -66,6 +112,13 @@ template <class Sc> __device__ __forceinline__ Sc divk(const Sc &a, int k) {
   if (k == 1) return a;
   if ((k & (k - 1)) == 0) return a * (1.0 / k);
   return divd(a, rcp_known((double)k, 1.0 / k));
+}
+// the same on doubles by div_known (k of two bits: exact for every dividend)
+__device__ __forceinline__ double divk(const double &a, int k) {
+  if (k == 1) return a;
+  if ((k & (k - 1)) == 0) return a * (1.0 / k);
+  return k == 3 ? div_known(a, 0x1.5555555555555p-2, 0x1.5555555555555p-56)
+                : div_known(a, 0x1.9999999999999p-3, 0x1.3333333333333p-56);  // k == 5
 }
 
 // divk for dividends of any magnitude (divr_any's range)

@@ -38,7 +38,23 @@ template <int ORD> struct Tables {
   double sigma;
   double wts[NG];                 // gllWts_ngll
   double ridl;                    // RN(1/idl[HS+1]), the bridge polynomial's divisor
+  // derived (host::complete_tables, awfl_recip.h): 1/idl[HS+1] = ridl_h + ridl_l, and the
+  // constants of the weights' mapping, d + d*d, 3d, d*d and 1 - 2d for d = idl[i]
+  double ridl_h, ridl_l;
+  double map_a[HS + 2], map_b[HS + 2], map_c[HS + 2], map_d[HS + 2];
 };
+
+// Entries of the ord-5 reconstruction tables that the FP64 kernels hold as literals
+// (compared with the tables when they are uploaded): the others are zero or a power of two
+// times one of these.
+constexpr double kW24 = 0x1.5555555555555p-5;     // 1/24
+constexpr double kW2324 = 0x1.eaaaaaaaaaaabp-1;   // 23/24
+constexpr double kW1312 = 0x1.1555555555555p+0;   // 13/12
+constexpr double kH00 = 0x1.3333333333333p-8;     // 3/640
+constexpr double kH10 = 0x1.eeeeeeeeeeeefp-5;     // 29/480
+constexpr double kH20 = 0x1.1c88888888889p+0;     // 1067/960
+constexpr double kH01 = 0x1.aaaaaaaaaaaabp-4;     // 5/48
+constexpr double kH11 = 0x1.6aaaaaaaaaaabp-1;     // 17/24
 
 // Per-line constants of one sweep.
 struct SweepArgs {
