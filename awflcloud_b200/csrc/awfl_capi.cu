@@ -30,6 +30,7 @@ struct awfl_ctx {
   int device = 0;
   int hs = 0, ngll = 0, sim2d = 0, dimswitch = 1, nsm = 148;
   double dx = 0, dy = 0, dz = 0;
+  double nrdx[3][2] = {};  // -1/dx, -1/dy, -1/dz as div_known's pairs (set_spacing)
   // tables (Spatial:274-315)
   std::vector<double> recon, c2g, s2g, deriv, idl, pts_ord, wts_ord, pts_ngll, wts_ngll;
   double sigma = 0;
@@ -357,11 +358,20 @@ SweepArgs sweep_args(awfl_ctx *c, void *state, void *tend, double dt, int dir, i
   A.weno_s = c->cfg.weno_scalars; A.weno_w = c->cfg.weno_winds; A.sim2d = c->sim2d; A.mode = mode;
   A.dxd = dir == 0 ? c->dx : (dir == 1 ? c->dy : c->dz);
   A.rdxd = 1.0 / A.dxd;
+  A.nrdx_h = c->nrdx[dir][0];
+  A.nrdx_l = c->nrdx[dir][1];
   A.dt = dt;
   A.plane = 0;
   A.dens_c = c->d_dens_c; A.denstheta_c = c->d_denstheta_c;
   A.dens_g = c->d_dens_g; A.denstheta_g = c->d_denstheta_g; A.pres_g = c->d_pres_g;
   return A;
+}
+
+// The grid spacing and what the FP64 sweeps divide by it with.
+void set_spacing(awfl_ctx *c, double dx, double dy, double dz) {
+  c->dx = dx; c->dy = dy; c->dz = dz;
+  const double d[3] = {dx, dy, dz};
+  for (int i = 0; i < 3; i++) host::split_recip(-d[i], &c->nrdx[i][0], &c->nrdx[i][1]);
 }
 
 bool bad_ptr(const void *p) { return p == nullptr || (reinterpret_cast<uintptr_t>(p) & 7) != 0; }
@@ -462,9 +472,7 @@ int awfl_create(const awfl_config *cfg, int device, awfl_ctx **out) {
   c->hs = hs;
   c->ngll = cfg->ord == 5 ? 3 : 5;
   c->sim2d = cfg->ny == 1;
-  c->dx = cfg->xlen / cfg->nx;
-  c->dy = cfg->ylen / cfg->ny;
-  c->dz = cfg->zlen / cfg->nz;
+  set_spacing(c, cfg->xlen / cfg->nx, cfg->ylen / cfg->ny, cfg->zlen / cfg->nz);
   build_tables(c);
   build_background(c);
   if (device < 0) {  // host-only context: tables and background, no device resources
@@ -846,7 +854,7 @@ int awfl_create_slab(const awfl_config *global, int nslabs, int slab, int device
   c->slab = slab;
   c->xoff = slab * base + (slab < extra ? slab : extra);
   c->nx_global = global->nx;
-  c->dx = global->xlen / global->nx;  // the grid's spacing, as the undivided grid computes it
+  set_spacing(c, global->xlen / global->nx, c->dy, c->dz);  // the grid's spacing, as the undivided grid computes it
   if (nslabs > 1) {
     const bool periodic = global->bc_x == AWFL_BC_PERIODIC;
     c->xlo_ex = periodic || slab > 0;

@@ -310,6 +310,45 @@ __device__ __forceinline__ void reconstruct_gll_any(const Sc (&sten)[ORD], Sc (&
   }
 }
 
+// x + y/k for a small positive integer k: y/k is exact for a power of two, so that on doubles
+// the sum is one FMA.
+template <class Sc> __device__ __forceinline__ Sc add_divk(const Sc &x, const Sc &y, int k) { return x + divk(y, k); }
+__device__ __forceinline__ double add_divk(const double &x, const double &y, int k) {
+  if ((k & (k - 1)) == 0) return __fma_rn(1.0 / k, y, x);
+  return x + divk(y, k);
+}
+
+// -(sum_s deriv(s, ii) x[s]) / dx / k: level k of a variable's time series from its flux x at
+// level k-1. On doubles the sum leaves out what changes at most the sign of a zero level
+// (which ends in sums that do not see it: the edge states start from level 0, never -0): the
+// leading 0 +, and at ord 5, whose matrix is {-3 4 -1; -1 0 1; 1 -4 3}, the products by 0
+// and +-1; a product by 4 is exact and goes into an FMA. The quotient is div_known's, a
+// power-of-two k folded into the divisor's pair.
+template <int ORD, class Sc>
+__device__ __forceinline__ Sc deriv_term(const Sc (&x)[OrdTraits<ORD>::NGLL], int ii, int k, const SweepArgs &A) {
+  constexpr int NG = OrdTraits<ORD>::NGLL;
+  const Tables<ORD> &T = tab<ORD>();
+  if constexpr (std::is_same<Sc, double>::value) {
+    double d;
+    if constexpr (ORD == 5) {
+      if (ii == 0) d = __fma_rn(4., x[1], -3. * x[0]) - x[2];
+      else if (ii == 1) d = x[2] - x[0];
+      else d = __fma_rn(-4., x[1], x[0]) + 3. * x[2];
+    } else {
+      d = T.deriv[ii] * x[0];
+#pragma unroll
+      for (int s = 1; s < NG; s++) d += T.deriv[s * NG + ii] * x[s];
+    }
+    if ((k & (k - 1)) == 0) return div_known(d, A.nrdx_h * (1.0 / k), A.nrdx_l * (1.0 / k));
+    return divk(div_known(d, A.nrdx_h, A.nrdx_l), k);
+  } else {
+    Sc d = 0.;
+#pragma unroll
+    for (int s = 0; s < NG; s++) d += T.deriv[s * NG + ii] * x[s];
+    return divk(divd(-d, rcp_known(A.dxd, A.rdxd)), k);
+  }
+}
+
 // Reconstruction + ADER differential transform + edge time average of one cell
 // (the K2 kernels: Spatial:665-811 x, 1028-1171 y, 1385-1552 z; diffTransformEulerConsX/Y/Z
 // at Spatial:1837-2091; compute_timeAvg[_edges] at Spatial:2130-2177).
@@ -366,15 +405,14 @@ __device__ __forceinline__ void cell_recon(const Sten &sten, int kb, const Sweep
   Sc g[NA][NG];
   Sc srcfill = 0;
   Rcp<Sc> rr[NG];  // the density of each GLL point: divisor of its velocities and products
-  const Rcp<double> rdx = rcp_known(A.dxd, A.rdxd);
 #pragma unroll
   for (int ii = 0; ii < NG; ii++) {
     const Sc r = q[idR][0][ii];
     rr[ii] = make_rcp<Sc>(r);
-    const Sc u = divr(q[idU][0][ii], rr[ii]);
-    const Sc v = divr(q[idV][0][ii], rr[ii]);
-    const Sc w = divr(q[idW][0][ii], rr[ii]);
-    const Sc t = divr(q[idT][0][ii], rr[ii]);
+    const Sc u = divp(q[idU][0][ii], rr[ii]);
+    const Sc v = divp(q[idV][0][ii], rr[ii]);
+    const Sc w = divp(q[idW][0][ii], rr[ii]);
+    const Sc t = divp(q[idT][0][ii], rr[ii]);
     const Sc vn = NM == 1 ? u : (NM == 2 ? v : w);
     f[0][0][ii] = r * vn * u;
     f[1][0][ii] = r * vn * v;
@@ -391,43 +429,25 @@ __device__ __forceinline__ void cell_recon(const Sten &sten, int kb, const Sweep
 #pragma unroll
     for (int ii = 0; ii < NG; ii++) sr[kt][ii] = srcfill;
 
-  // diffTransformEulerCons{X,Y,Z}
-#pragma unroll
-  for (int kt = 1; kt < NA; kt++)
-#pragma unroll
-    for (int ii = 0; ii < NG; ii++) {
-      f[0][kt][ii] = 0; f[1][kt][ii] = 0; f[2][kt][ii] = 0; f[3][kt][ii] = 0;
-      g[kt][ii] = 0;
-    }
+  // diffTransformEulerCons{X,Y,Z}. Level kt+1 of f and g is still zero where the reference's
+  // Cauchy products read it: those terms are left out.
 #pragma unroll
   for (int kt = 0; kt < NA - 1; kt++) {
+    Sc fl[5][NG];  // the flux of each variable
+#pragma unroll
+    for (int s = 0; s < NG; s++) {
+      fl[idR][s] = q[NM][kt][s];
+#pragma unroll
+      for (int m = 1; m <= 4; m++) fl[m][s] = f[m - 1][kt][s];
+      if (DIR == 2 && kt == 0) fl[NM][s] = fl[NM][s] + C0 * g[kt][s] - A.pres_g[kb * NG + s];
+      else fl[NM][s] = add_divk(fl[NM][s], C0 * g[kt][s], kt == 0 ? 1 : 2);
+    }
 #pragma unroll
     for (int ii = 0; ii < NG; ii++) {
-      Sc dq[5] = {0., 0., 0., 0., 0.};
 #pragma unroll
-      for (int s = 0; s < NG; s++) {
-        const double D = T.deriv[s * NG + ii];
-        dq[idR] += D * (q[NM][kt][s]);
-#pragma unroll
-        for (int m = 1; m <= 3; m++) {
-          if (m == NM) {
-            if (DIR == 2 && kt == 0) {
-              dq[m] += D * (f[m - 1][kt][s] + C0 * g[kt][s] - A.pres_g[kb * NG + s]);
-            } else if (kt == 0) {
-              dq[m] += D * (f[m - 1][kt][s] + C0 * g[kt][s]);
-            } else {
-              dq[m] += D * (f[m - 1][kt][s] + C0 * g[kt][s] / 2);
-            }
-          } else {
-            dq[m] += D * (f[m - 1][kt][s]);
-          }
-        }
-        dq[idT] += D * (f[3][kt][s]);
-      }
-#pragma unroll
-      for (int m = 0; m < 5; m++) q[m][kt + 1][ii] = divk(divd(-dq[m], rdx), kt + 1);
+      for (int m = 0; m < 5; m++) q[m][kt + 1][ii] = deriv_term<ORD>(fl[m], ii, kt + 1, A);
       if (DIR == 2) {
-        q[idW][kt + 1][ii] = divk(divd(-dq[idW], rdx), kt + 1) + divk(sr[kt][ii], kt + 1);
+        q[idW][kt + 1][ii] = add_divk(q[idW][kt + 1][ii], sr[kt][ii], kt + 1);
         if (A.bc == BC_WALL) {
           if (kb == A.nz - 1) q[idW][kt + 1][NG - 1] = 0;
           if (kb == 0) q[idW][kt + 1][0] = 0;
@@ -437,20 +457,23 @@ __device__ __forceinline__ void cell_recon(const Sten &sten, int kb, const Sweep
     }
 #pragma unroll
     for (int ii = 0; ii < NG; ii++) {
-      Sc tot[4] = {0., 0., 0., 0.};
+      Sc tot[4];
 #pragma unroll
-      for (int ir = 0; ir <= kt + 1; ir++) {
+      for (int x = 0; x < 4; x++) tot[x] = q[NM][0][ii] * q[x + 1][kt + 1][ii];
+#pragma unroll
+      for (int ir = 1; ir <= kt + 1; ir++) {
 #pragma unroll
         for (int x = 0; x < 4; x++)
           tot[x] += q[NM][ir][ii] * q[x + 1][kt + 1 - ir][ii] - q[idR][ir][ii] * f[x][kt + 1 - ir][ii];
       }
 #pragma unroll
-      for (int x = 0; x < 4; x++) f[x][kt + 1][ii] = divr(tot[x], rr[ii]);
-      Sc tg = 0.;
+      for (int x = 0; x < 4; x++) f[x][kt + 1][ii] = divp(tot[x], rr[ii]);
+      const Sc g0 = GAMMA * g[0][ii] * q[idT][kt + 1][ii];
+      Sc tg = (kt + 1.) * g0;
 #pragma unroll
-      for (int ir = 0; ir <= kt; ir++)
+      for (int ir = 1; ir <= kt; ir++)
         tg += (kt + 1. - ir) * (GAMMA * g[ir][ii] * q[idT][kt + 1 - ir][ii] - q[idT][ir][ii] * g[kt + 1 - ir][ii]);
-      g[kt + 1][ii] = (GAMMA * g[0][ii] * q[idT][kt + 1][ii] + divk(tg, kt + 1)) / q[idT][0][ii];
+      g[kt + 1][ii] = (g0 + divk(tg, kt + 1)) / q[idT][0][ii];
     }
   }
   rec.series(q);
@@ -461,8 +484,8 @@ __device__ __forceinline__ void cell_recon(const Sten &sten, int kb, const Sweep
     double dtmult = A.dt;
 #pragma unroll
     for (int kt = 1; kt < NA; kt++) {
-      l += divk(q[v][kt][0] * dtmult, kt + 1);
-      r += divk(q[v][kt][NG - 1] * dtmult, kt + 1);
+      l = add_divk(l, q[v][kt][0] * dtmult, kt + 1);
+      r = add_divk(r, q[v][kt][NG - 1] * dtmult, kt + 1);
       dtmult *= A.dt;
     }
     eL[v] = l;
@@ -474,7 +497,7 @@ __device__ __forceinline__ void cell_recon(const Sten &sten, int kb, const Sweep
 #pragma unroll
     for (int kt = 1; kt < NA; kt++) {
 #pragma unroll
-      for (int ii = 0; ii < NG; ii++) sr[0][ii] += divk(sr[kt][ii] * dtmult, kt + 1);
+      for (int ii = 0; ii < NG; ii++) sr[0][ii] = add_divk(sr[0][ii], sr[kt][ii] * dtmult, kt + 1);
       dtmult *= A.dt;
     }
     Sc sa = 0.;
@@ -503,10 +526,10 @@ __device__ __forceinline__ void riemann(const Sc (&qL)[5], const Sc (&qR)[5], in
     t = 0.5 * (qL[4] + qR[4]);
   } else {
     const Rcp<Sc> rl = make_rcp<Sc>(qL[0]), rg = make_rcp<Sc>(qR[0]);
-    vel[0] = 0.5 * (divr(qL[1], rl) + divr(qR[1], rg));
-    vel[1] = 0.5 * (divr(qL[2], rl) + divr(qR[2], rg));
-    vel[2] = 0.5 * (divr(qL[3], rl) + divr(qR[3], rg));
-    t = 0.5 * (divr(qL[4], rl) + divr(qR[4], rg));
+    vel[0] = 0.5 * (divp(qL[1], rl) + divp(qR[1], rg));
+    vel[1] = 0.5 * (divp(qL[2], rl) + divp(qR[2], rg));
+    vel[2] = 0.5 * (divp(qL[3], rl) + divp(qR[3], rg));
+    t = 0.5 * (divp(qL[4], rl) + divp(qR[4], rg));
   }
   const Sc p = C0 * pow_gamma(r * t);
   const Sc cs2 = GAMMA * p / r;
@@ -515,16 +538,16 @@ __device__ __forceinline__ void riemann(const Sc (&qL)[5], const Sc (&qR)[5], in
   const Rcp<Sc> rt = make_rcp<Sc>(t), rt2 = rcp_twice(rt), rc2 = make_rcp<Sc>(2. * cs);
   Sc w1, w2, w3;
   if (vn > 0) {
-    w1 = qL[0] - divr(qL[4], rt);
-    w2 = qL[QA] - divr(va * qL[4], rt);
-    w3 = qL[QB] - divr(vb * qL[4], rt);
+    w1 = qL[0] - divp(qL[4], rt);
+    w2 = qL[QA] - divp(va * qL[4], rt);
+    w3 = qL[QB] - divp(vb * qL[4], rt);
   } else {
-    w1 = qR[0] - divr(qR[4], rt);
-    w2 = qR[QA] - divr(va * qR[4], rt);
-    w3 = qR[QB] - divr(vb * qR[4], rt);
+    w1 = qR[0] - divp(qR[4], rt);
+    w2 = qR[QA] - divp(va * qR[4], rt);
+    w3 = qR[QB] - divp(vb * qR[4], rt);
   }
-  const Sc w5 = divr(vn * qR[0], rc2) - divr(qR[QN], rc2) + divr(qR[4], rt2);
-  const Sc w6 = divr(-vn * qL[0], rc2) + divr(qL[QN], rc2) + divr(qL[4], rt2);
+  const Sc w5 = divp(vn * qR[0], rc2) - divp(qR[QN], rc2) + divp(qR[4], rt2);
+  const Sc w6 = divp(-vn * qL[0], rc2) + divp(qL[QN], rc2) + divp(qL[4], rt2);
   Sc q[5];
   q[0] = w1 + w5 + w6;
   q[QN] = vn * w1 + (vn - cs) * w5 + (vn + cs) * w6;
@@ -533,10 +556,10 @@ __device__ __forceinline__ void riemann(const Sc (&qL)[5], const Sc (&qR)[5], in
   q[4] = t * w5 + t * w6;
   const Rcp<Sc> r0 = make_rcp<Sc>(q[0]);
   F[0] = q[QN];
-  F[QN] = divr(q[QN] * q[QN], r0) + C0 * pow_gamma(q[4]);
-  F[QA] = divr(q[QN] * q[QA], r0);
-  F[QB] = divr(q[QN] * q[QB], r0);
-  F[4] = divr(q[QN] * q[4], r0);
+  F[QN] = divp(q[QN] * q[QN], r0) + C0 * pow_gamma(q[4]);
+  F[QA] = divp(q[QN] * q[QA], r0);
+  F[QB] = divp(q[QN] * q[QB], r0);
+  F[4] = divp(q[QN] * q[4], r0);
   if (DIR == 2) {  // Spatial:1628-1629
     if (kf < A.nz) F[idW] -= A.pres_g[kf * NG + 0];
     if (kf == A.nz) F[idW] -= A.pres_g[(A.nz - 1) * NG + NG - 1];

@@ -66,6 +66,7 @@ struct SweepArgs {
   int weno_s, weno_w, sim2d, mode;
   double dxd;      // dx, dy or dz
   double rdxd;     // RN(1/dxd)
+  double nrdx_h, nrdx_l;  // -1/dxd = nrdx_h + nrdx_l (div_known's pair, awfl_recip.h)
   double dt;
   const double *dens_c, *denstheta_c;             // hyDensCells, hyDensThetaCells (nz+2hs)
   const double *dens_g, *denstheta_g, *pres_g;    // hyDensGLL, hyDensThetaGLL, hyPressureGLL (nz*ngll)

@@ -66,7 +66,7 @@ struct P64Trc : P64 {
         }
       // RN(1 / density) of the GLL points (the sweep's own reciprocals, rr in cell_recon)
 #pragma unroll
-      for (int ii = 0; ii < NG; ii++) base[(2 * NS + 1 + ii) * n + cell] = 1.0 / q[idR][0][ii];
+      for (int ii = 0; ii < NG; ii++) base[(2 * NS + 1 + ii) * n + cell] = make_rcp<double>(q[idR][0][ii]).y;
     }
   };
   template <int ORD, int DIR, class S>
@@ -91,13 +91,13 @@ struct P64Trc : P64 {
     constexpr int NM = 1 + DIR;
     const long n = (long)A.nx * A.ny * A.nz, nfm = (long)(A.nx + 1) * (A.ny + 1) * (A.nz + 1);
     double *fr = A.tend + trc_cell_planes<NG>() * n + face;
-    const double vn = DIR == 1 ? 0.5 * (qL[NM] + qR[NM]) : 0.5 * (qL[NM] / qL[0] + qR[NM] / qR[0]);
+    const double vn = DIR == 1 ? 0.5 * (qL[NM] + qR[NM]) : 0.5 * (divp(qL[NM], make_rcp<double>(qL[0])) + divp(qR[NM], make_rcp<double>(qR[0])));
     fr[0] = F[0];
     fr[nfm] = vn;
     fr[2 * nfm] = 0.5 * (qL[NM] + qR[NM]);
     const double rup = vn > 0 ? qL[0] : qR[0];
     fr[3 * nfm] = rup;
-    fr[4 * nfm] = 1.0 / rup;  // RN(1/rup): the tracer fluxes' shared divisor
+    fr[4 * nfm] = make_rcp<double>(rup).y;  // RN(1/rup): the tracer fluxes' shared divisor
   }
 };
 
