@@ -78,10 +78,6 @@ struct P64Rec : P64 {
   template <int ORD, int DIR, class S>
   static __device__ __forceinline__ void recon(const S &sten, int kb, const Args &A, double (&eL)[5],
                                                double (&eR)[5], double &src, long cell) {
-    if (cell < 0) {  // the periodic prologue's repeat of cell L-1: recorded in its chunk
-      cell_recon<ORD, DIR>(sten, kb, A, eL, eR, src);
-      return;
-    }
     constexpr int NG = OrdTraits<ORD>::NGLL;
     const long n = (long)A.nx * A.ny * A.nz;
     cell_recon<ORD, DIR>(sten, kb, A, eL, eR, src, Rec<ORD>{A.tend, n, cell});
@@ -94,6 +90,7 @@ struct P64Rec : P64 {
   }
 };
 template <int ORD, int DIR> struct PolicyShape<P64Rec, ORD, DIR> : PolicyShape<P64, ORD, DIR> {};
+template <int ORD, int DIR> struct PolicyShapes<P64Rec, ORD, DIR> : SmallShapes<ORD, DIR> {};
 
 cudaError_t launch_sweep_rec(int ord, int dir, const SweepArgs &A, cudaStream_t st) {
   return launch_sweep_any<P64Rec>(ord, dir, A, st);

@@ -329,6 +329,7 @@ SweepArgs32 sweep_args32(awfl_ctx *c, void *state, void *tend, double dt, int di
   A.nx = c->cfg.nx; A.ny = c->cfg.ny; A.nz = c->cfg.nz;
   A.bc = dir == 0 ? c->cfg.bc_x : (dir == 1 ? c->cfg.bc_y : c->cfg.bc_z);
   A.weno_s = c->cfg.weno_scalars; A.weno_w = c->cfg.weno_winds; A.sim2d = c->sim2d; A.mode = mode;
+  A.nsm = c->nsm;
   A.inv_dxd = (float)(1.0 / (dir == 0 ? c->dx : (dir == 1 ? c->dy : c->dz)));
   A.dt = (float)dt;
   A.bg = c->bg32;
@@ -356,6 +357,7 @@ SweepArgs sweep_args(awfl_ctx *c, void *state, void *tend, double dt, int dir, i
   A.nx = c->cfg.nx; A.ny = c->cfg.ny; A.nz = c->cfg.nz;
   A.bc = dir == 0 ? c->cfg.bc_x : (dir == 1 ? c->cfg.bc_y : c->cfg.bc_z);
   A.weno_s = c->cfg.weno_scalars; A.weno_w = c->cfg.weno_winds; A.sim2d = c->sim2d; A.mode = mode;
+  A.nsm = c->nsm;
   A.dxd = dir == 0 ? c->dx : (dir == 1 ? c->dy : c->dz);
   A.rdxd = 1.0 / A.dxd;
   A.nrdx_h = c->nrdx[dir][0];

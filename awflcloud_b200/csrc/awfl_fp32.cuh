@@ -511,6 +511,9 @@ struct P32 {
   }
   static constexpr int min_blocks(int) { return 1; }  // forcing more CTAs per SM measured slower
   using Args = SweepArgs32;
+  // rows that TMA cannot address (16-byte pitch) come by cp.async: 107 instead of about 85 us
+  // for the x split of 130x100x70
+  static double base_factor(const Args &A) { return A.nx % 4 ? 1.25 : 1.0; }
   // the Kahan compensations of the cell's five variables, loaded before the reconstruction
   struct Aux {
     float c[5];
@@ -555,6 +558,14 @@ struct P32 {
 // z 4 x 32 (y/z: a warp = 8 lines x 4 positions, 32-byte row segments).
 template <> struct PolicyShape<P32, 5, 0> { static constexpr int C = 8, W = 16; };
 template <> struct PolicyShape<P32, 5, 1> { static constexpr int C = 4, W = 32; };
+
+// The shapes for small grids (PolicyShapes, awfl_sweep.cuh).
+template <int DIR> struct PolicyShapes<P32, 5, DIR> {
+  static constexpr int n = 4;
+  static constexpr int C[4] = {DIR == 0 ? 4 : 8, 16, 32, 128}, W[4] = {DIR == 0 ? 32 : 16, 8, 4, 1};
+  static constexpr double factor[4] = {DIR == 0 ? 1.0 : (DIR == 1 ? 1.05 : 1.1), DIR == 0 ? 1.15 : (DIR == 1 ? 1.2 : 1.3),
+                                       DIR == 0 ? 1.25 : (DIR == 1 ? 1.7 : 1.8), DIR == 0 ? 1.5 : 2.5};
+};
 
 // Uploads the FP32 tables into this translation unit's constant memory.
 static inline cudaError_t upload_tables32_here(int ord, const double *recon, const double *c2g, const double *s2g,

@@ -24,6 +24,7 @@ struct SweepArgs32 {
   float *tend;
   int nx, ny, nz;
   int bc, weno_s, weno_w, sim2d, mode;
+  int nsm;       // SMs of the device (the launch picks the tile shape by it)
   float inv_dxd;
   float dt;
   Bg32 bg;

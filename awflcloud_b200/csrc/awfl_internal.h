@@ -64,6 +64,7 @@ struct SweepArgs {
   int nx, ny, nz;
   int bc;          // BC along the sweep direction
   int weno_s, weno_w, sim2d, mode;
+  int nsm;         // SMs of the device (the launch picks the tile shape by it)
   double dxd;      // dx, dy or dz
   double rdxd;     // RN(1/dxd)
   double nrdx_h, nrdx_l;  // -1/dxd = nrdx_h + nrdx_l (div_known's pair, awfl_recip.h)

@@ -36,6 +36,7 @@ struct P64 {
 #endif
   static constexpr int min_blocks(int ord) { return ord == 5 ? AWFL_P64_MIN_BLOCKS_ORD5 : 1; }
   using Args = SweepArgs;
+  static double base_factor(const Args &) { return 1.0; }
   struct Aux {};
   static __device__ __forceinline__ void load_aux(const Args &, long, long, Aux &) {}
 
@@ -99,5 +100,14 @@ struct P64 {
 template <> struct PolicyShape<P64, 5, 0> { static constexpr int C = AWFL_P64_XC, W = AWFL_P64_XW; };
 template <> struct PolicyShape<P64, 5, 1> { static constexpr int C = AWFL_P64_YC, W = AWFL_P64_YW; };
 template <> struct PolicyShape<P64, 5, 2> { static constexpr int C = AWFL_P64_ZC, W = AWFL_P64_ZW; };
+
+// The shapes for small grids, x, y and z alike (PolicyShapes, awfl_sweep.cuh).
+template <int ORD, int DIR> struct SmallShapes { static constexpr int n = 0; };
+template <int DIR> struct SmallShapes<5, DIR> {
+  static constexpr int n = 3;
+  static constexpr int C[3] = {DIR == 0 ? 8 : 16, 32, 128}, W[3] = {DIR == 0 ? 16 : 8, 4, 1};
+  static constexpr double factor[3] = {1.0, 1.0, 1.1};
+};
+template <int ORD, int DIR> struct PolicyShapes<P64, ORD, DIR> : SmallShapes<ORD, DIR> {};
 
 }  // namespace awfl

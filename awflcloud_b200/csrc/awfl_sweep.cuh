@@ -32,8 +32,8 @@
 // time average), the face flux, the tendency and the in-place update:
 //   using Real; using Args;                         Args has state/tend/nx/ny/nz/bc/mode/sim2d
 //   template <int ORD, int DIR, class S> recon(sten, kb, A, eL[5], eR[5], src, cell)
-//                                          (cell: the cell's (k,j,i) index, -1 for the
-//                                          periodic prologue's repeat of cell L-1)
+//                                          (cell: the cell's (k,j,i) index, -1 for a
+//                                          cell of a neighbouring slab)
 //   template <int DIR, int NG>            flux(qL[5], qR[5], kf, A, F[5])
 //                                          (kf: the face's k for z, the line's k for x, y)
 //   template <int DIR>                    tendency(v, Fl, Fr, src, A) -> Real
@@ -48,10 +48,12 @@
 //                                          global memory for ensembles)
 //   min_blocks(ORD)                        CTAs per SM the register budget must allow
 //   kSlab                                  the policy runs x splits of slabs (A.xh)
+//   base_factor(A)                         (host) what keeps PolicyShape from its usual speed
 //   load(A, gidx) / store(A, gidx, x)      state element access (halo writes)
 //   store_tend(A, tidx, x)                 tendency output (MODE_TEND)
 #pragma once
 
+#include <algorithm>
 #include <type_traits>
 
 #include "awfl_internal.h"
@@ -118,6 +120,19 @@ template <class T> __device__ __forceinline__ T shfl_up_any(const T &x, int delt
   return y;
 }
 
+// the value of lane `lane` of the segment, likewise
+template <class T> __device__ __forceinline__ T shfl_idx_any(const T &x, int lane, int width) {
+  static_assert(sizeof(T) % 4 == 0, "shuffled types are made of 4-byte words");
+  constexpr int N = (int)(sizeof(T) / 4);
+  unsigned u[N];
+  __builtin_memcpy(u, &x, sizeof(T));
+#pragma unroll
+  for (int i = 0; i < N; i++) u[i] = __shfl_sync(0xffffffffu, u[i], lane, width);
+  T y;
+  __builtin_memcpy(&y, u, sizeof(T));
+  return y;
+}
+
 // orders this thread's generic-proxy shared-memory accesses before later async-proxy ones
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
 
@@ -147,7 +162,10 @@ template <class P> struct PolicyFaceRec<P, std::void_t<decltype(P::kFaceRec)>> :
 // SLAB: the x sweep of a slab of a larger grid, whose ends may take their halo values from
 // the neighbouring slabs (A.xh); a separate instantiation, so that the plain sweeps carry
 // none of its registers.
-template <class P, int ORD, int DIR, int C, int W, bool TMA = false, bool SLAB = false>
+// ENDS: the line's last face takes a spare lane (below): for the small-grid shapes, since
+// the large grids' sweeps, with many chunks to a line, lose more by the registers (FP32:
+// 146 instead of 126, three CTAs per SM instead of four).
+template <class P, int ORD, int DIR, int C, int W, bool TMA = false, bool SLAB = false, bool ENDS = false>
 __device__ __forceinline__ void sweep_tile(const typename P::Args &A, const int bx, const int by,
                                            const void *tmap = nullptr) {
   using Real = typename P::Real;
@@ -193,19 +211,22 @@ __device__ __forceinline__ void sweep_tile(const typename P::Args &A, const int 
   __shared__ __align__(128) Real ring[5][R * RW];
   __shared__ __align__(8) unsigned long long mbar;  // TMA path only
   __shared__ int sAbort;                            // TMA path: a wait of this tile gave up
-  __shared__ Real sEL[5][(C + 1) * W];
-  __shared__ Real sER[5][(C + 1) * W];
-  __shared__ Real sF[5][(C + 1) * W];
-  __shared__ Real sSrc[DIR == 2 ? (C + 1) * W : 1];
+  constexpr int ES = SHFL ? 1 : C + 1;  // edge slots of a line: the carry alone, or every face
+  __shared__ Real sEL[5][ES * W];
+  __shared__ Real sER[5][ES * W];
+  __shared__ Real sF[5][ES * W];
+  __shared__ Real sSrc[DIR == 2 ? ES * W : 1];
   __shared__ Real sWrap[5][HS * W];
   __shared__ Real sEL0[5][W];
+  __shared__ Real sF1[5][W];  // periodic lines: the flux of face 1 and the source of cell 0
+  __shared__ Real sSrc0[DIR == 2 ? W : 1];
 
   const int tid = threadIdx.y * blockDim.x + threadIdx.x;
   // position in chunk, line within CTA
   const int c = DIR == 0 ? (int)threadIdx.x : (SHFL ? (tid & (C - 1)) : (int)threadIdx.y);
   const int w = DIR == 0 ? (int)threadIdx.y : (SHFL ? tid / C : (int)threadIdx.x);
   // edge/flux slot (0..C) of this line: consecutive threads of a warp hit consecutive words
-  auto E = [&](int slot) { return DIR == 0 ? w * (C + 1) + slot : slot * W + w; };
+  auto E = [&](int slot) { return DIR == 0 ? w * ES + slot : slot * W + w; };
 
   const int nx = A.nx, ny = A.ny, nz = A.nz;
   const long sx = 1, sy = nx + 2 * HS, sz = (long)(ny + 2 * HS) * sy, sv = (long)(nz + 2 * HS) * sz;
@@ -273,13 +294,16 @@ __device__ __forceinline__ void sweep_tile(const typename P::Args &A, const int 
     if (periodic) return first ? G(v, q) : sWrap[v][q * W + w];
     return v == NM ? Real(0) : G(v, L - 1);
   };
-  auto finish = [&](int cell, const Real *Fl, const Real *Fr, Real sa, const typename P::Aux &aux) {
+  auto finish_as = [&](int cell, auto orig, const Real *Fl, const Real *Fr, Real sa, const typename P::Aux &aux) {
 #pragma unroll
     for (int v = 0; v < 5; v++) {
       const Real tnd = P::template tendency<DIR>(v, Fl[v], Fr[v], sa, A);
-      if (A.mode == MODE_APPLY) P::apply(A, lb + v * sv + cell * sd, ringAt(v, cell), tnd, aux, v);
+      if (A.mode == MODE_APPLY) P::apply(A, lb + v * sv + cell * sd, orig(v), tnd, aux, v);
       else P::store_tend(A, tb + v * tv + cell * tsd, tnd);
     }
+  };
+  auto finish = [&](int cell, const Real *Fl, const Real *Fr, Real sa, const typename P::Aux &aux) {
+    finish_as(cell, [&](int v) -> Real { return ringAt(v, cell); }, Fl, Fr, sa, aux);
   };
   // a row value into its ring slot: asynchronously when it is a load of an interior cell
   auto stage = [&](int v, int p, bool first) {
@@ -346,29 +370,52 @@ __device__ __forceinline__ void sweep_tile(const typename P::Args &A, const int 
       for (int v = 0; v < 5; v++) pre[v] = p < L ? G(v, p) : topval(v, p, true);
     }
   }
-  // periodic: the left state of face 0 is the right edge of cell L-1; a slab bordering
-  // another below: the right edge of that slab's last cell (position -1)
-  if (valid && (periodic || xlo) && c == 0) {
+  // A periodic line's face 0 is its face L: its left state, the right edge of cell L-1, is
+  // known when the line ends, so the flux of face 0 and the update of cell 0 wait until
+  // then (cell 0's right flux and source are kept, its original value is in the wrap rows).
+  // The sweep used to reconstruct cell L-1 a second time up front, on one lane of C: 1/L
+  // more work, and a whole chunk's latency per tile (FP64 ord 9, 128x128x64: 2.91 -> 2.66 ms
+  // per step; FP32 ord 9: 0.76 -> 0.64).
+  const bool late0 = periodic && !xlo;
+  // a periodic line's cell 0 from the states and the flux of face L: the same states as face
+  // 0, so the same flux, but for z's per-face background
+  auto finish_first = [&](const Real (&qL)[5], const Real (&qR)[5], const Real (&FL)[5]) {
+    Real F[5], F1[5];
+#pragma unroll
+    for (int v = 0; v < 5; v++) {
+      F[v] = FL[v];
+      F1[v] = sF1[v][w];
+    }
+    if constexpr (DIR == 2) P::template flux<DIR, NG>(qL, qR, 0, A, F);
+    if constexpr (PolicyFaceRec<P>::value) P::template face_rec<ORD, DIR>(A, fb, DIR == 2 ? 0 : kline, qL, qR, F);
+    typename P::Aux aux;
+    if (A.mode == MODE_APPLY) P::load_aux(A, lb, sv, aux);
+    finish_as(0, [&](int v) -> Real { return sWrap[v][w]; }, F, F1, DIR == 2 ? sSrc0[w] : Real(0), aux);
+  };
+  // a slab bordering another below: the left state of face 0 is the right edge of that
+  // slab's last cell (position -1)
+  if constexpr (SLAB) if (valid && xlo && c == 0) {
     auto wrapSten = [&](int v, int m) -> Real {
-      if (xlo) {
-        const int p = -1 - HS + m;
-        return p < 0 ? XH(0, v, p + HS + 1) : G(v, p);
-      }
-      int p = L - 1 - HS + m;
-      p %= L;
-      if (p < 0) p += L;
-      return G(v, p);
+      const int p = -1 - HS + m;
+      return p < 0 ? XH(0, v, p + HS + 1) : G(v, p);
     };
     Real eL[5], eR[5], sa;
-    P::template recon<ORD, DIR>(wrapSten, DIR == 2 ? L - 1 : kline, A, eL, eR, sa, -1L);
+    P::template recon<ORD, DIR>(wrapSten, kline, A, eL, eR, sa, -1L);
 #pragma unroll
     for (int v = 0; v < 5; v++) sER[v][E(0)] = eR[v];
   }
 
   const int nchunk = (L + C - 1) / C;
+  // ENDS: face L takes a lane of its own in the last chunk where that has one to spare, so
+  // that the line ends with the chunk instead of one more flux on one lane of C (the
+  // epilogue; a third of a short line's time). A periodic x or y line of one full chunk has its faces
+  // 0 and L as one: lane 0 takes it, its left state from the last lane (ROT).
+  const bool ends = ENDS && L % C != 0 && !xhi;
+  const bool rot = ENDS && SHFL && DIR != 2 && late0 && L == C;
   for (int t = 0; t < nchunk; t++) {
     const int base = t * C;
     const int nvalid = min(C, L - base);
+    const int nface = nvalid + (ends && t + 1 == nchunk ? 1 : 0);  // faces base .. of this chunk
     if constexpr (TMA) {
       // the chunk's boxes have landed; a wait that gives up flags the error and ends the
       // tile's use of TMA (the rest of the tile's chunks come by cp.async)
@@ -402,7 +449,8 @@ __device__ __forceinline__ void sweep_tile(const typename P::Args &A, const int 
     }
     // the compensation (or other per-cell input) of the cell this thread updates below
     typename P::Aux aux;
-    if (valid && c < nvalid && base + c >= 1 && A.mode == MODE_APPLY) P::load_aux(A, lb + (base + c - 1) * sd, sv, aux);
+    if (valid && c < nface && (rot || base + c >= 1) && A.mode == MODE_APPLY)
+      P::load_aux(A, lb + (rot && c == 0 ? L - 1 : base + c - 1) * sd, sv, aux);
     // next chunk's rows (stored into the ring at the next (A); the updates of this chunk
     // never reach them)
     if (EARLY_PREFETCH && valid && t + 1 < nchunk) {
@@ -434,40 +482,70 @@ __device__ __forceinline__ void sweep_tile(const typename P::Args &A, const int 
       }
     }
     if constexpr (SHFL) {
-      const bool act = valid && c < nvalid;
-      // face base+c: left state = right edge of cell base+c-1 (the lane below, or the carry)
+      const bool act = valid && c < nface;
+      // face base+c: left state = right edge of cell base+c-1 (the lane below, or the carry;
+      // ROT: lane 0 takes the last lane's)
       Real qL[5], F[5];
 #pragma unroll
       for (int v = 0; v < 5; v++) {
         const Real up = shfl_up_any(eR[v], 1, C);
         qL[v] = c == 0 ? sER[v][E(0)] : up;
       }
-      if (act) {
+      if (rot) {
+#pragma unroll
+        for (int v = 0; v < 5; v++) {
+          const Real top = shfl_idx_any(eR[v], C - 1, C);
+          if (c == 0) qL[v] = top;
+        }
+      }
+      if (ENDS && nface > nvalid) {
+        __syncwarp();  // sEL0 may be this chunk's
+        if (c == nvalid) {
+#pragma unroll
+          for (int v = 0; v < 5; v++) eL[v] = late0 ? sEL0[v][w] : qL[v];
+        }
+      }
+      if (act && (rot || !(late0 && base + c == 0))) {
         if (base + c == 0 && !periodic && !xlo) {
 #pragma unroll
           for (int v = 0; v < 5; v++) qL[v] = eL[v];
         }
         P::template flux<DIR, NG>(qL, eL, DIR == 2 ? base + c : kline, A, F);
-        if constexpr (PolicyFaceRec<P>::value)
+        if constexpr (PolicyFaceRec<P>::value) {
           P::template face_rec<ORD, DIR>(A, fb + (base + c) * fsd, DIR == 2 ? base + c : kline, qL, eL, F);
+          if (rot && c == 0) P::template face_rec<ORD, DIR>(A, fb + L * fsd, kline, qL, eL, F);
+        }
       } else {
 #pragma unroll
         for (int v = 0; v < 5; v++) F[v] = Real(0);
       }
       // cell base+c-1: its left face's flux from the lane below (or the carry), its right
-      // face's from this lane
+      // face's from this lane; ROT: lane 0 finishes cell L-1
       Real Fl[5];
 #pragma unroll
       for (int v = 0; v < 5; v++) {
         const Real up = shfl_up_any(F[v], 1, C);
         Fl[v] = c == 0 ? sF[v][E(0)] : up;
       }
+      if (rot) {
+#pragma unroll
+        for (int v = 0; v < 5; v++) {
+          const Real top = shfl_idx_any(F[v], C - 1, C);
+          if (c == 0) Fl[v] = top;
+        }
+      }
       Real sl = Real(0);  // z: the source term of cell base+c-1
       if constexpr (DIR == 2) {
         const Real up = shfl_up_any(sa, 1, C);
         sl = c == 0 ? sSrc[E(0)] : up;
       }
-      if (act && base + c >= 1) finish(base + c - 1, Fl, F, sl, aux);
+      if (act && late0 && !rot && base + c == 1) {
+#pragma unroll
+        for (int v = 0; v < 5; v++) sF1[v][w] = F[v];
+        if (DIR == 2) sSrc0[w] = sl;
+      } else if (act && (rot || base + c >= 1)) {
+        finish(rot && c == 0 ? L - 1 : base + c - 1, Fl, F, sl, aux);
+      }
       if (!ASYNC && valid && t + 1 < nchunk) {
         const int p = base + C + HS + c;
 #pragma unroll
@@ -482,15 +560,17 @@ __device__ __forceinline__ void sweep_tile(const typename P::Args &A, const int 
         }
         if (DIR == 2) sSrc[E(0)] = sa;
       }
+      if constexpr (ENDS)
+        if (late0 && act && c == nvalid) finish_first(qL, eL, F);  // the lane of face L
       __syncwarp();
       continue;
     }
     __syncthreads();  // (B)
-    if (valid && c < nvalid) {
+    if (valid && c < nface && !(late0 && base + c == 0)) {
       const int f = base + c;  // face index = left face of cell f
       Real qL[5], qR[5], F[5];
 #pragma unroll
-      for (int v = 0; v < 5; v++) qR[v] = sEL[v][E(c)];
+      for (int v = 0; v < 5; v++) qR[v] = c < nvalid ? sEL[v][E(c)] : (late0 ? sEL0[v][w] : sER[v][E(c)]);
 #pragma unroll
       for (int v = 0; v < 5; v++) qL[v] = (f == 0 && !periodic && !xlo) ? qR[v] : sER[v][E(c)];
       P::template flux<DIR, NG>(qL, qR, DIR == 2 ? f : kline, A, F);
@@ -499,7 +579,7 @@ __device__ __forceinline__ void sweep_tile(const typename P::Args &A, const int 
       for (int v = 0; v < 5; v++) sF[v][E(c + 1)] = F[v];
     }
     __syncthreads();  // (C)
-    if (valid && c < nvalid) {
+    if (valid && c < nface) {
       const int cell = base + c - 1;
       if (cell >= 0) {
         Real Fl[5], Fr[5];
@@ -508,7 +588,13 @@ __device__ __forceinline__ void sweep_tile(const typename P::Args &A, const int 
           Fl[v] = sF[v][E(c)];
           Fr[v] = sF[v][E(c + 1)];
         }
-        finish(cell, Fl, Fr, DIR == 2 ? sSrc[E(c)] : Real(0), aux);
+        if (late0 && cell == 0) {
+#pragma unroll
+          for (int v = 0; v < 5; v++) sF1[v][w] = Fr[v];
+          if (DIR == 2) sSrc0[w] = sSrc[E(c)];
+        } else {
+          finish(cell, Fl, Fr, DIR == 2 ? sSrc[E(c)] : Real(0), aux);
+        }
       }
     }
     if (!ASYNC && !EARLY_PREFETCH && valid && t + 1 < nchunk) {
@@ -517,6 +603,16 @@ __device__ __forceinline__ void sweep_tile(const typename P::Args &A, const int 
       for (int v = 0; v < 5; v++) pre[v] = p < L ? G(v, p) : topval(v, p, false);
     }
     __syncthreads();  // (D)
+    if (ENDS && late0 && valid && c == nvalid && nface > nvalid) {  // the lane of face L
+      Real qL[5], qR[5], F[5];
+#pragma unroll
+      for (int v = 0; v < 5; v++) {
+        qL[v] = sER[v][E(nvalid)];
+        qR[v] = sEL0[v][w];
+        F[v] = sF[v][E(nvalid + 1)];
+      }
+      finish_first(qL, qR, F);
+    }
     if (valid && c == 0) {
 #pragma unroll
       for (int v = 0; v < 5; v++) {
@@ -526,8 +622,9 @@ __device__ __forceinline__ void sweep_tile(const typename P::Args &A, const int 
       if (DIR == 2) sSrc[E(0)] = sSrc[E(nvalid)];
     }
   }
-  // ---- epilogue: face L and the last cell (same thread that wrote the carry)
-  if (valid && c == 0) {
+  // ---- epilogue, where no lane was left for it: face L and the last cell (same thread that
+  // wrote the carry), then a periodic line's face 0 and cell 0
+  if (valid && c == 0 && !ends && !rot) {
     Real qL[5], qR[5], F[5], Fl[5];
 #pragma unroll
     for (int v = 0; v < 5; v++) {
@@ -550,6 +647,7 @@ __device__ __forceinline__ void sweep_tile(const typename P::Args &A, const int 
     typename P::Aux aux;
     if (A.mode == MODE_APPLY) P::load_aux(A, lb + (L - 1) * sd, sv, aux);
     finish(L - 1, Fl, F, DIR == 2 ? sSrc[E(0)] : Real(0), aux);
+    if (late0) finish_first(qL, qR, F);
   }
   if constexpr (TMA) {  // every issued phase has completed (or been given up on, flagged)
     __syncthreads();
@@ -567,18 +665,25 @@ __device__ __forceinline__ void sweep_tile(const typename P::Args &A, const int 
 // CTAs per SM the register budget must allow: the policy's figure, or for the x-slab
 // sweeps of ord 5 at least AWFL_SLAB_MINB_ORD5 (4: the FP32 slab sweep drops from 142 to
 // 112 registers, no spills, and its x split of a 128x256x128 slab from 0.442 to 0.408 ms;
-// the same bound on the single-grid FP32 sweeps made them slower)
+// the same bound on the single-grid FP32 sweeps made them slower), and so for the
+// small-grid shapes
 #ifndef AWFL_SLAB_MINB_ORD5
 #define AWFL_SLAB_MINB_ORD5 4
 #endif
-template <class P, int ORD, bool SLAB> constexpr int sweep_min_blocks() {
-  return (SLAB && ORD == 5 && AWFL_SLAB_MINB_ORD5 > P::min_blocks(ORD)) ? AWFL_SLAB_MINB_ORD5 : P::min_blocks(ORD);
+template <class P, int ORD, bool CAP> constexpr int sweep_min_blocks() {
+  return (CAP && ORD == 5 && AWFL_SLAB_MINB_ORD5 > P::min_blocks(ORD)) ? AWFL_SLAB_MINB_ORD5 : P::min_blocks(ORD);
 }
 
-template <class P, int ORD, int DIR, int C, int W, bool TMA, bool SLAB = false>
-__global__ void __launch_bounds__(C *W, (sweep_min_blocks<P, ORD, SLAB>())) sweep_kernel(const __grid_constant__ typename P::Args A) {
-  if constexpr (TMA) sweep_tile<P, ORD, DIR, C, W, true, SLAB>(A, blockIdx.x, blockIdx.y, P::tma_map(A));
-  else sweep_tile<P, ORD, DIR, C, W, false, SLAB>(A, blockIdx.x, blockIdx.y);
+template <class P, int ORD, int DIR, int C, int W, bool TMA, bool SLAB = false, bool ENDS = false>
+__global__ void __launch_bounds__(C *W, (sweep_min_blocks<P, ORD, SLAB || ENDS>())) sweep_kernel(const __grid_constant__ typename P::Args A) {
+  if constexpr (TMA) sweep_tile<P, ORD, DIR, C, W, true, SLAB, ENDS>(A, blockIdx.x, blockIdx.y, P::tma_map(A));
+  else sweep_tile<P, ORD, DIR, C, W, false, SLAB, ENDS>(A, blockIdx.x, blockIdx.y);
+}
+template <class P, int ORD, int DIR, int C, int W, bool TMA, bool SLAB, bool ENDS>
+cudaError_t launch_sweep_kernel(const typename P::Args &A, dim3 grid, cudaStream_t st) {
+  const dim3 block(DIR == 0 ? C : W, DIR == 0 ? W : C);
+  sweep_kernel<P, ORD, DIR, C, W, TMA, SLAB, ENDS><<<grid, block, 0, st>>>(A);
+  return cudaGetLastError();
 }
 
 template <int ORD, int DIR> struct SweepShape;
@@ -595,39 +700,78 @@ template <class P, int ORD, int DIR> struct PolicyShape : SweepShape<ORD, DIR> {
 
 // Policies with wider elements (P::kWdiv > 1) use fewer lines per CTA to stay within the
 // 48 KB of static shared memory.
-template <class P, int ORD, int DIR, int C = PolicyShape<P, ORD, DIR>::C,
-          int W = (PolicyShape<P, ORD, DIR>::W / P::kWdiv > 0 ? PolicyShape<P, ORD, DIR>::W / P::kWdiv : 1)>
-cudaError_t launch_sweep_t(const typename P::Args &A, cudaStream_t st) {
-  dim3 block(DIR == 0 ? C : W, DIR == 0 ? W : C);
+template <class P, int ORD, int DIR, int C, int W>
+cudaError_t launch_sweep_shape(const typename P::Args &A, cudaStream_t st) {
   dim3 grid;
   if (DIR == 0) grid = dim3((A.ny + W - 1) / W, A.nz);
   else if (DIR == 1) grid = dim3((A.nx + W - 1) / W, A.nz);
   else grid = dim3((A.nx + W - 1) / W, A.ny);
+  constexpr bool base = C == PolicyShape<P, ORD, DIR>::C;
   // the x split of a slab with neighbouring slabs' columns: the SLAB instantiation
-  if constexpr (DIR == 0 && P::kSlab) {
-    if (A.xh[0] != nullptr || A.xh[1] != nullptr) {
-      if constexpr (P::kTmaRing) {
-        typename P::Args a = A;
-        if (P::prepare_tma(a, ORD, DIR, C, W)) {
-          sweep_kernel<P, ORD, DIR, C, W, true, true><<<grid, block, 0, st>>>(a);
-          return cudaGetLastError();
-        }
-      }
-      sweep_kernel<P, ORD, DIR, C, W, false, true><<<grid, block, 0, st>>>(A);
-      return cudaGetLastError();
-    }
-  }
-  if constexpr (P::kTmaRing) {
+  bool slab = false;
+  if constexpr (DIR == 0 && P::kSlab && base) slab = A.xh[0] != nullptr || A.xh[1] != nullptr;
+  if constexpr (P::kTmaRing && (DIR == 0 || W % 4 == 0)) {
     // the policy encodes this launch's tensor map (box = one chunk of one variable); a
     // layout TMA cannot address (alignment) leaves tma off and the cp.async path runs
     typename P::Args a = A;
     if (P::prepare_tma(a, ORD, DIR, C, W)) {
-      sweep_kernel<P, ORD, DIR, C, W, true><<<grid, block, 0, st>>>(a);
-      return cudaGetLastError();
+      if constexpr (DIR == 0 && P::kSlab && base)
+        if (slab) return launch_sweep_kernel<P, ORD, DIR, C, W, true, true, false>(a, grid, st);
+      return launch_sweep_kernel<P, ORD, DIR, C, W, true, false, !base>(a, grid, st);
     }
   }
-  sweep_kernel<P, ORD, DIR, C, W, false><<<grid, block, 0, st>>>(A);
-  return cudaGetLastError();
+  if constexpr (DIR == 0 && P::kSlab && base)
+    if (slab) return launch_sweep_kernel<P, ORD, DIR, C, W, false, true, false>(A, grid, st);
+  return launch_sweep_kernel<P, ORD, DIR, C, W, false, false, !base>(A, grid, st);
+}
+
+// Time of a sweep of `tiles` CTAs marching along lines of L cells in chunks of C, in units of
+// the chunk latency of an SM's only CTA: ceil(L/C) chunks, and an epilogue where no lane of
+// the last one is free, each as long as the CTAs that share an SM make it. Measured with the
+// FP64 ord-5 sweep: 5.9 us for one CTA per SM, 8 for two, 10.5 for three, 13 for four, the
+// most; the tiles of a grid take equally long, so an SM runs its share four at a time.
+inline double sweep_cost(int C, int L, long tiles, int nsm, bool ends) {
+  const long k = (tiles + nsm - 1) / nsm;  // of the busiest SM
+  return ((L + C - 1) / C + (ends && L % C ? 0.0 : 0.35)) * (k / 4 * 2.2 + (k % 4 ? 0.6 + 0.4 * (k % 4) : 0.0));
+}
+
+// The single-grid sweep of a policy whose PolicyShapes lists further shapes takes its first
+// one (PolicyShape, the best on large grids) unless another is 5% cheaper by sweep_cost
+// times its own factor: a small grid has too few lines to fill the chip W at a time, and
+// marches along them in ceil(L/C) dependent chunks, so it wants more cells of a line at once
+// (C up to 128) and fewer lines per CTA. The factor is what a shape's narrower rows (y, z:
+// W elements) or its barriers (C > 32) cost on a full chip. Measured, us for the x, y and z
+// splits, PolicyShape -> the rule: FP64 32x32x16 18.6 32.9 22.7 -> 13.8 14.4 14.6, 64x64x32
+// 37.3 57.7 43.3 -> 35.2 37.2 37.8, 97x61x45 (walls) 78.4 90.7 75.8 -> 76.5 62.0 72.2,
+// 400x1x200 150 - 190 -> 37.3 - 28.9; FP32 64x64x32 25.0 43.3 29.0 -> 16.8 20.8 18.9,
+// 97x61x45 39.4 49.6 41.5 -> 33.4 25.2 31.2, 400x1x200 120 - 129 -> 18.6 - 18.7.
+template <class P, int ORD, int DIR, class = void> struct PolicyShapes { static constexpr int n = 0; };
+
+template <class P, int ORD, int DIR>
+cudaError_t launch_sweep_t(const typename P::Args &A, cudaStream_t st) {
+  using B = PolicyShape<P, ORD, DIR>;
+  constexpr int BW = B::W / P::kWdiv > 0 ? B::W / P::kWdiv : 1;
+  using S = PolicyShapes<P, ORD, DIR>;
+  if constexpr (S::n > 0) {
+    const int L = DIR == 0 ? A.nx : (DIR == 1 ? A.ny : A.nz);
+    const int across = DIR == 0 ? A.ny : A.nx;  // lines of one plane, W to a tile
+    const long planes = DIR == 2 ? A.ny : A.nz;
+    int best = -1;
+    double cost = 0.95 * P::base_factor(A) * sweep_cost(B::C, L, (across + BW - 1) / BW * planes, A.nsm, false);
+    for (int i = 0; i < S::n; i++) {
+      const double c = S::factor[i] * sweep_cost(S::C[i], L, (across + S::W[i] - 1) / S::W[i] * planes, A.nsm, true);
+      if (c < cost) { best = i; cost = c; }
+    }
+    if constexpr (DIR == 0 && P::kSlab) {
+      if (A.xh[0] != nullptr || A.xh[1] != nullptr) best = -1;
+    }
+    if constexpr (S::n > 0) if (best == 0) return launch_sweep_shape<P, ORD, DIR, S::C[0], S::W[0]>(A, st);
+    if constexpr (S::n > 1) if (best == 1) return launch_sweep_shape<P, ORD, DIR, S::C[1], S::W[1]>(A, st);
+    if constexpr (S::n > 2) if (best == 2) return launch_sweep_shape<P, ORD, DIR, S::C[2], S::W[2]>(A, st);
+    if constexpr (S::n > 3) if (best == 3) return launch_sweep_shape<P, ORD, DIR, S::C[3], S::W[3]>(A, st);
+    static_assert(S::n <= 4, "shape dispatch");
+  }
+  return launch_sweep_shape<P, ORD, DIR, B::C, BW>(A, st);
 }
 
 template <class P>

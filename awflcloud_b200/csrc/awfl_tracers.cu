@@ -72,10 +72,6 @@ struct P64Trc : P64 {
   template <int ORD, int DIR, class S>
   static __device__ __forceinline__ void recon(const S &sten, int kb, const Args &A, double (&eL)[5],
                                                double (&eR)[5], double &src, long cell) {
-    if (cell < 0) {  // the periodic prologue's repeat of cell L-1: recorded in its chunk
-      cell_recon<ORD, DIR>(sten, kb, A, eL, eR, src);
-      return;
-    }
     constexpr int NG = OrdTraits<ORD>::NGLL;
     constexpr int HS = (ORD - 1) / 2;
     const long n = (long)A.nx * A.ny * A.nz;
@@ -102,6 +98,7 @@ struct P64Trc : P64 {
 };
 
 template <int ORD, int DIR> struct PolicyShape<P64Trc, ORD, DIR> : PolicyShape<P64, ORD, DIR> {};
+template <int ORD, int DIR> struct PolicyShapes<P64Trc, ORD, DIR> : SmallShapes<ORD, DIR> {};
 
 namespace {
 

@@ -62,10 +62,6 @@ struct P32Trc : P32 {
   template <int ORD, int DIR, class S>
   static __device__ __forceinline__ void recon(const S &sten, int kb, const Args &A, float (&eL)[5], float (&eR)[5],
                                                float &src, long cell) {
-    if (cell < 0) {  // the periodic prologue's repeat of cell L-1: recorded in its chunk
-      cell_recon32<ORD, DIR>(sten, kb, A, eL, eR, src);
-      return;
-    }
     constexpr int NG = OrdTraits<ORD>::NGLL;
     constexpr int HS = (ORD - 1) / 2;
     const long n = (long)A.nx * A.ny * A.nz;
