@@ -105,7 +105,15 @@ struct F2 {
   __device__ __forceinline__ explicit F2(float c) : v(make_float2(c, c)) {}
 };
 __device__ __forceinline__ F2 operator+(F2 a, F2 b) { return F2(__fadd2_rn(a.v, b.v)); }
-__device__ __forceinline__ F2 operator-(F2 a, F2 b) { return F2(__fadd2_rn(a.v, make_float2(-b.v.x, -b.v.y))); }
+__device__ __forceinline__ F2 operator-(F2 a, F2 b) {  // FADD2 with a negated operand (no intrinsic for it)
+  unsigned long long x, y, z;
+  __builtin_memcpy(&x, &a.v, 8);
+  __builtin_memcpy(&y, &b.v, 8);
+  asm("sub.rn.ftz.f32x2 %0, %1, %2;" : "=l"(z) : "l"(x), "l"(y));
+  F2 r;
+  __builtin_memcpy(&r.v, &z, 8);
+  return r;
+}
 __device__ __forceinline__ F2 operator*(F2 a, F2 b) { return F2(__fmul2_rn(a.v, b.v)); }
 __device__ __forceinline__ F2 operator*(float c, F2 b) { return F2(__fmul2_rn(make_float2(c, c), b.v)); }
 __device__ __forceinline__ F2 operator*(F2 a, float c) { return F2(__fmul2_rn(a.v, make_float2(c, c))); }
@@ -120,9 +128,6 @@ __device__ __forceinline__ F2 fmaT(F2 a, F2 b, F2 c) { return F2(__ffma2_rn(a.v,
 __device__ __forceinline__ F2 fmaT(F2 a, float b, F2 c) { return F2(__ffma2_rn(a.v, make_float2(b, b), c.v)); }
 __device__ __forceinline__ float rcpT(float x) { return frcp(x); }
 __device__ __forceinline__ F2 rcpT(F2 x) { return F2(frcp(x.v.x), frcp(x.v.y)); }
-__device__ __forceinline__ float divT(float a, float b) { return __fdividef(a, b); }
-__device__ __forceinline__ F2 divT(float a, F2 b) { return F2(__fdividef(a, b.v.x), __fdividef(a, b.v.y)); }
-__device__ __forceinline__ F2 divT(F2 a, F2 b) { return F2(__fdividef(a.v.x, b.v.x), __fdividef(a.v.y, b.v.y)); }
 
 template <int N> __device__ __forceinline__ F2 tv_evalf2(const F2 *a) {
   if constexpr (N == 3) return awfl_tv_n3<F2>(a);
@@ -177,7 +182,7 @@ __device__ __forceinline__ void weno_coefs32(const T (&u)[ORD], T (&aw)[ORD]) {
   T sum = T(0.f);
 #pragma unroll
   for (int i = 0; i < HS + 2; i++) {
-    wts[i] = divT(Tb.idl[i], fmaT(tv[i], tv[i], T(eps)));
+    wts[i] = Tb.idl[i] * rcpT(fmaT(tv[i], tv[i], T(eps)));
     sum += wts[i];
   }
   T inv = rcpT(sum + eps);
@@ -186,9 +191,8 @@ __device__ __forceinline__ void weno_coefs32(const T (&u)[ORD], T (&aw)[ORD]) {
   for (int i = 0; i < HS + 2; i++) {
     const T w = wts[i] * inv;
     const float d = Tb.idl[i];
-    const T num = w * ((d + d * d) + (w * w - (3.f * d) * w));
-    const T den = (d * d) + w * (1.f - 2.f * d);
-    wts[i] = divT(num, den);
+    const T num = w * fmaT(w, w + (-3.f * d), T(d + d * d));
+    wts[i] = num * rcpT(fmaT(w, 1.f - 2.f * d, T(d * d)));
     sum += wts[i];
   }
   inv = rcpT(sum + eps);
@@ -204,11 +208,77 @@ __device__ __forceinline__ void weno_coefs32(const T (&u)[ORD], T (&aw)[ORD]) {
     }
   }
 }
+// Ideal weights and relaxation of ord 5 (WenoLimiter.h:28-90) as compile-time constants (the
+// uploaded tables are compared with them), and what the routine below derives from them.
+namespace w5 {
+constexpr double kSum = 2 * 1. + 73.564225445964 + 1584.89319246111;
+// the weights of the side parabolas, of the centred one and of the bridge polynomial
+constexpr double kD0 = 1. / kSum, kD1 = 73.564225445964 / kSum, kD3 = 1584.89319246111 / kSum;
+constexpr double kSigma = 0.73564225445964;
+// the bridge polynomial (quartic minus the idl-weighted parabolas, over idl[3]) in the
+// differences below: e0 = E0S*S + E01*s1, h1 = c + H1*g, h2 = H2S*S + H21*s1, h3 = H3*g,
+// h4 = H4*(S - 2 s1)
+constexpr double kE0S = (3. / 640 + kD0 / 24) / kD3, kE01 = (-1. / 24 - 6. / 640 + kD1 / 24) / kD3;
+constexpr double kH1 = (-5. / 48 + kD0 / 2) / kD3;
+constexpr double kH2S = (-1. / 16 - kD0 / 2) / kD3, kH21 = (.625 - kD1 / 2) / kD3;
+constexpr double kH3 = 1 / (12 * kD3), kH4 = 1 / (24 * kD3);
+}  // namespace w5
+
+// The ord-5 WENO reconstruction to the three GLL points in differences of the stencil: with
+// d_i = u[i+1]-u[i] and s_i = d[i+1]-d[i], the three parabolas are u[2] - s_i/24 + a_i x +
+// (s_i/2) x^2 and the bridge polynomial has the few coefficients of w5, where the matrix
+// form (weno_coefs32) multiplies 49 entries. Equal in exact arithmetic, the weights summing
+// to one; about 100 FP32 instructions instead of 150, and u[2] enters the values unrounded.
+// The sweep is issue-bound: with the time series on point pairs
+// (Pts below), 1,500 -> 1,130 instructions per cell and split, 256x256x128 step 1.433 -> 1.200 ms.
+template <class T> __device__ __forceinline__ void weno_gll5(const T (&u)[5], T (&out)[3]) {
+  using namespace w5;
+  const T d0 = u[1] - u[0], d1 = u[2] - u[1], d2 = u[3] - u[2], d3 = u[4] - u[3];
+  const T s0 = d1 - d0, s1 = d2 - d1, s2 = d3 - d2;
+  const T a0 = fmaT(.5f, s0, d1), c = fmaT(.5f, s1, d1), a2 = fmaT(-.5f, s2, d2);
+  const T S = s0 + s2, g = s2 - s0;
+  const T e0 = fmaT((float)kE0S, S, (float)kE01 * s1);
+  const T h1 = fmaT((float)kH1, g, c);
+  const T h2 = fmaT((float)kH2S, S, (float)kH21 * s1);
+  const T h3 = (float)kH3 * g;
+  const T h4 = fmaT((float)kH4, S, (float)(-2 * kH4) * s1);
+  // smoothness indicators (coefs_to_tv of the parabolas and of the bridge polynomial)
+  const float k13 = (float)(13. / 12);
+  const T t0 = fmaT(a0, a0, (k13 * s0) * s0), t1 = fmaT(c, c, (k13 * s1) * s1), t2 = fmaT(a2, a2, (k13 * s2) * s2);
+  T t3 = fmaT(h1, fmaT(.5f, h3, h1), (39.1125f * h3) * h3);
+  t3 = fmaT(h2, fmaT(4.2f, h4, (float)(13. / 3) * h2), t3);
+  t3 = fmaT(625.8f * h4, h4, t3);
+  const T avg = (t0 + t1 + t2) * (float)(1. / 3);
+  t3 = fmaT(t3 - avg, (float)kSigma, avg);
+  // weights idl/(tv^2 + eps), up to the common factor idl[0] that the normalisation drops
+  const T eps = T(1.0e-20f);
+  T w[4] = {rcpT(fmaT(t0, t0, eps)), (float)(kD1 / kD0) * rcpT(fmaT(t1, t1, eps)), rcpT(fmaT(t2, t2, eps)),
+            (float)(kD3 / kD0) * rcpT(fmaT(t3, t3, eps))};
+  T inv = rcpT(((w[0] + w[1]) + (w[2] + w[3])) + eps);
+#pragma unroll
+  for (int i = 0; i < 4; i++) {  // map_weights (WenoLimiter.h:12-17)
+    const double d = i == 1 ? kD1 : (i == 3 ? kD3 : kD0);
+    const T x = w[i] * inv;
+    w[i] = (x * fmaT(x, x + (float)(-3 * d), T((float)(d + d * d)))) * rcpT(fmaT(x, (float)(1 - 2 * d), T((float)(d * d))));
+  }
+  inv = rcpT(((w[0] + w[1]) + (w[2] + w[3])) + eps);
+  const T Q = fmaT(w[0], s0, fmaT(w[1], s1, w[2] * s2));
+  const T P = fmaT(w[0], a0, fmaT(w[1], c, fmaT(w[2], a2, w[3] * fmaT(.25f, h3, h1))));
+  const T mid = fmaT(inv, fmaT((float)(-1. / 24), Q, w[3] * e0), u[2]);
+  const T ev = fmaT(inv, fmaT(.125f, Q, w[3] * fmaT(.0625f, h4, .25f * h2)), mid);
+  const T od = (.5f * inv) * P;
+  out[0] = ev - od;
+  out[1] = mid;
+  out[2] = ev + od;
+}
+
 template <int ORD, class T>
 __device__ __forceinline__ void reconstruct_gll32(const T (&sten)[ORD], T (&out)[OrdTraits<ORD>::NGLL], bool doweno) {
   constexpr int NG = OrdTraits<ORD>::NGLL;
   const Tables32<ORD> &Tb = tab32<ORD>();
-  if (doweno) {
+  if (ORD == 5 && doweno) {
+    if constexpr (ORD == 5) weno_gll5(sten, out);
+  } else if (doweno) {
     T wc[ORD];
     weno_coefs32<ORD>(sten, wc);
     // polynomial coefficients -> values at the GLL points, which sit symmetrically about
@@ -238,9 +308,98 @@ __device__ __forceinline__ void reconstruct_gll32(const T (&sten)[ORD], T (&out)
   }
 }
 
+// (1+x)^gamma - 1 on two lanes
+__device__ __forceinline__ F2 binom_gamma_m1(F2 x) {
+  if (fmaxf(fabsf(x.v.x), fabsf(x.v.y)) < 0.05f) {
+    F2 p = fmaT(F2((float)kB6), x, F2((float)kB5));
+    p = fmaT(p, x, F2((float)kB4));
+    p = fmaT(p, x, F2((float)kB3));
+    p = fmaT(p, x, F2((float)kB2));
+    p = fmaT(p, x, F2((float)kB1));
+    return p * x;
+  }
+  return F2(binom_gamma_m1(x.v.x), binom_gamma_m1(x.v.y));
+}
+
+// The values of one quantity at a cell's GLL points: the mirror points (ii, NG-1-ii) as the
+// two lanes of the paired FP32 instructions, the centre alone. All points of a cell go
+// through the same operations, so the time series takes 2 instructions where it took 3 (ord
+// 5; 3 for 5 at ord 9), with no lane to broadcast.
+template <int NG> struct Pts {
+  F2 p[NG / 2];
+  float c;
+  __device__ __forceinline__ float get(int ii) const {
+    return ii == NG / 2 ? c : (ii < NG / 2 ? p[ii].v.x : p[NG - 1 - ii].v.y);
+  }
+  __device__ __forceinline__ void set(int ii, float x) {
+    if (ii == NG / 2) c = x;
+    else if (ii < NG / 2) p[ii].v.x = x;
+    else p[NG - 1 - ii].v.y = x;
+  }
+};
+template <int NG, class F> __device__ __forceinline__ Pts<NG> each(const F &f) {
+  Pts<NG> r;
+#pragma unroll
+  for (int i = 0; i < NG / 2; i++) r.p[i] = f([i](const Pts<NG> &x) -> const F2 & { return x.p[i]; });
+  r.c = f([](const Pts<NG> &x) -> const float & { return x.c; });
+  return r;
+}
+template <int NG> __device__ __forceinline__ Pts<NG> operator+(const Pts<NG> &a, const Pts<NG> &b) {
+  return each<NG>([&](auto e) { return e(a) + e(b); });
+}
+template <int NG> __device__ __forceinline__ Pts<NG> operator*(const Pts<NG> &a, const Pts<NG> &b) {
+  return each<NG>([&](auto e) { return e(a) * e(b); });
+}
+template <int NG> __device__ __forceinline__ Pts<NG> operator*(float a, const Pts<NG> &b) {
+  return each<NG>([&](auto e) { return a * e(b); });
+}
+template <int NG> __device__ __forceinline__ Pts<NG> operator-(const Pts<NG> &a, const Pts<NG> &b) {
+  return each<NG>([&](auto e) { return e(a) - e(b); });
+}
+template <int NG> __device__ __forceinline__ Pts<NG> fmaT(const Pts<NG> &a, const Pts<NG> &b, const Pts<NG> &c) {
+  return each<NG>([&](auto e) { return fmaT(e(a), e(b), e(c)); });
+}
+template <int NG> __device__ __forceinline__ Pts<NG> fmaT(float a, const Pts<NG> &b, const Pts<NG> &c) {
+  return each<NG>([&](auto e) { return fmaT(a, e(b), e(c)); });
+}
+template <int NG> __device__ __forceinline__ Pts<NG> rcpT(const Pts<NG> &a) {
+  return each<NG>([&](auto e) { return rcpT(e(a)); });
+}
+template <int NG> __device__ __forceinline__ Pts<NG> binom_gamma_m1(const Pts<NG> &a) {
+  return each<NG>([&](auto e) { return binom_gamma_m1(e(a)); });
+}
+template <int NG> __device__ __forceinline__ Pts<NG> same(float x) {
+  return each<NG>([&](auto e) { return std::decay_t<decltype(e(Pts<NG>()))>(x); });
+}
+// sum_s deriv(s, ii) x[s], times sc, at every point (the matrix has no centre weight at the
+// centre; at ord 5 it is {-3 4 -1; -1 0 1; 1 -4 3})
+template <int ORD> __device__ __forceinline__ Pts<OrdTraits<ORD>::NGLL> deriv32(const Pts<OrdTraits<ORD>::NGLL> &x, float sc) {
+  constexpr int NG = OrdTraits<ORD>::NGLL;
+  Pts<NG> r;
+  if constexpr (ORD == 5) {
+    const float x0 = x.get(0), x1 = x.c, x2 = x.get(2);
+    r.set(0, fmaf(4.f, x1, fmaf(-3.f, x0, -x2)));
+    r.set(1, x2 - x0);
+    r.set(2, fmaf(-4.f, x1, fmaf(3.f, x2, x0)));
+  } else {
+    const Tables32<ORD> &T = tab32<ORD>();
+#pragma unroll
+    for (int ii = 0; ii < NG; ii++) {
+      float acc = 0.f;
+#pragma unroll
+      for (int s = 0; s < NG; s++) {
+        if (ii == NG / 2 && s == NG / 2) continue;
+        acc = fmaf(T.deriv[s * NG + ii], x.get(s), acc);
+      }
+      r.set(ii, acc);
+    }
+  }
+  return sc * r;
+}
+
 // A recorder that keeps nothing (the default of cell_recon32): rec.series32(q, rtot) sees
-// the whole ADER series q[v][kt][ii] (level 0 as perturbations) and the total density of
-// the GLL points before the edge time average, for the tracer transport.
+// the whole ADER series q[v][kt] (level 0 as perturbations) and the total density of the GLL
+// points before the edge time average, for the tracer transport.
 struct NoRecord32 {
   template <class Q, class Rt> __device__ __forceinline__ void series32(const Q &, const Rt &) const {}
 };
@@ -252,9 +411,10 @@ __device__ __forceinline__ void cell_recon32(const Sten &sten, int kb, const Swe
   constexpr int NG = OrdTraits<ORD>::NGLL;
   constexpr int NA = NG;
   constexpr int NM = 1 + DIR;
+  using V = Pts<NG>;
   const Tables32<ORD> &T = tab32<ORD>();
 
-  float q[5][NA][NG];  // level 0: rho' (perturbation), rho*u/v/w, (rho*theta)' (perturbation)
+  V q[5][NA];  // level 0: rho' (perturbation), rho*u/v/w, (rho*theta)' (perturbation)
   // (rho', (rho theta)') and (rho u, rho v) in pairs on the paired FP32 instructions
 #pragma unroll
   for (int pr = 0; pr < 2; pr++) {
@@ -265,148 +425,116 @@ __device__ __forceinline__ void cell_recon32(const Sten &sten, int kb, const Swe
     reconstruct_gll32<ORD>(s2, o2, pr == 0 ? A.weno_s : A.weno_w);
 #pragma unroll
     for (int ii = 0; ii < NG; ii++) {
-      q[va][0][ii] = o2[ii].v.x;
-      q[vb][0][ii] = o2[ii].v.y;
+      q[va][0].set(ii, o2[ii].v.x);
+      q[vb][0].set(ii, o2[ii].v.y);
     }
   }
   {
-    float s[ORD];
+    float s[ORD], o[NG];
 #pragma unroll
     for (int m = 0; m < ORD; m++) s[m] = sten(idW, m);
-    reconstruct_gll32<ORD>(s, q[idW][0], A.weno_w);
-  }
-  if (DIR == 2 && A.bc == BC_WALL) {  // Spatial:1413-1416
-    if (kb == A.nz - 1) q[idW][0][NG - 1] = 0.f;
-    if (kb == 0) q[idW][0][0] = 0.f;
-  }
-  float rtot[NG], rttot[NG], Pbg[NG];
-  float f[4][NA][NG];
-  float g[NA][NG];  // (rho theta)^gamma series / (rho theta)_h^gamma
+    reconstruct_gll32<ORD>(s, o, A.weno_w);
 #pragma unroll
-  for (int ii = 0; ii < NG; ii++) {
-    float rb, rtb, irtb;
-    if (DIR == 2) {
-      rb = A.bg.rho_g[kb * NG + ii]; rtb = A.bg.rt_g[kb * NG + ii];
-      irtb = A.bg.irt_g[kb * NG + ii]; Pbg[ii] = A.bg.p_g[kb * NG + ii];
-    } else {
-      rb = A.bg.rho_c[HS + kb]; rtb = A.bg.rt_c[HS + kb];
-      irtb = A.bg.irt_c[HS + kb]; Pbg[ii] = A.bg.p_c[HS + kb];
+    for (int ii = 0; ii < NG; ii++) q[idW][0].set(ii, o[ii]);
+  }
+  const bool wall0 = DIR == 2 && A.bc == BC_WALL && kb == 0, wallN = DIR == 2 && A.bc == BC_WALL && kb == A.nz - 1;
+  auto wall = [&](V &w) {  // Spatial:1413-1416
+    if (wallN) w.set(NG - 1, 0.f);
+    if (wall0) w.set(0, 0.f);
+  };
+  if (DIR == 2) wall(q[idW][0]);
+  V rb, rtb, irtb, Pbg;  // background
+  if (DIR == 2) {
+#pragma unroll
+    for (int ii = 0; ii < NG; ii++) {
+      rb.set(ii, A.bg.rho_g[kb * NG + ii]);
+      rtb.set(ii, A.bg.rt_g[kb * NG + ii]);
+      irtb.set(ii, A.bg.irt_g[kb * NG + ii]);
+      Pbg.set(ii, A.bg.p_g[kb * NG + ii]);
     }
-    rtot[ii] = rb + q[idR][0][ii];
-    rttot[ii] = rtb + q[idT][0][ii];
-    const float ir = frcp(rtot[ii]);
-    const float vel[3] = {q[idU][0][ii] * ir, q[idV][0][ii] * ir, q[idW][0][ii] * ir};
-    const float th = rttot[ii] * ir;
-    const float rvn = q[NM][0][ii];  // r * vn
-    f[0][0][ii] = rvn * vel[0];
-    f[1][0][ii] = rvn * vel[1];
-    f[2][0][ii] = rvn * vel[2];
-    f[3][0][ii] = rvn * th;
-    g[0][ii] = binom_gamma_m1(q[idT][0][ii] * irtb);  // B(x); the scaled series starts at 1 + B
+  } else {
+    rb = same<NG>(A.bg.rho_c[HS + kb]);
+    rtb = same<NG>(A.bg.rt_c[HS + kb]);
+    irtb = same<NG>(A.bg.irt_c[HS + kb]);
+    Pbg = same<NG>(A.bg.p_c[HS + kb]);
   }
-  // z gravity source: every entry holds the kk = ngll-1 value (Spatial:1439), -(rho')*g
-  float sr[NA][NG];
-  const float srcfill = DIR == 2 ? -q[idR][0][NG - 1] * GRAVF : 0.f;
+  const V rtot = rb + q[idR][0], rttot = rtb + q[idT][0];
+  const V ir = rcpT(rtot);
+  V f[4][NA];
+  V g[NA];  // (rho theta)^gamma series / (rho theta)_h^gamma
 #pragma unroll
-  for (int kt = 0; kt < NA; kt++)
-#pragma unroll
-    for (int ii = 0; ii < NG; ii++) sr[kt][ii] = srcfill;
+  for (int m = 1; m <= 3; m++) f[m - 1][0] = q[NM][0] * (q[m][0] * ir);
+  f[3][0] = q[NM][0] * (rttot * ir);
+  g[0] = binom_gamma_m1(q[idT][0] * irtb);  // B(x); the scaled series starts at 1 + B
+  // z gravity source: every entry of the first level holds the kk = ngll-1 value (Spatial:1439)
+  const float srcfill = DIR == 2 ? -q[idR][0].get(NG - 1) * GRAVF : 0.f;
+  float sa = srcfill;  // its time average, GLL-weighted (the weights sum to one)
+  float dtm = A.dt;
 
   // diffTransformEulerCons{X,Y,Z} (Spatial:1837-2091)
 #pragma unroll
   for (int kt = 0; kt < NA - 1; kt++) {
+    const float sc = -A.inv_dxd * (1.0f / (kt + 1));
+    q[idR][kt + 1] = deriv32<ORD>(q[NM][kt], sc);
 #pragma unroll
-    for (int ii = 0; ii < NG; ii++) {
-      float dq[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+    for (int m = 1; m <= 4; m++) {
+      V fl = f[m - 1][kt];
+      if (m == NM) fl = fmaT(kt == 0 ? Pbg : 0.5f * Pbg, g[kt], fl);
+      q[m][kt + 1] = deriv32<ORD>(fl, sc);
+    }
+    if (DIR == 2) {
+      if (kt == 0) q[idW][1] = q[idW][1] + same<NG>(srcfill);
+      else q[idW][kt + 1] = fmaT(-GRAVF / (kt + 1), q[idR][kt], q[idW][kt + 1]);
+      wall(q[idW][kt + 1]);
+      float w = 0.f;
 #pragma unroll
-      for (int s = 0; s < NG; s++) {
-        if (ii == NG / 2 && s == NG / 2) continue;  // d/dx at the centre: no centre weight
-        const float D = T.deriv[s * NG + ii];
-        dq[idR] = fmaf(D, q[NM][kt][s], dq[idR]);
-#pragma unroll
-        for (int m = 1; m <= 3; m++) {
-          float fm = f[m - 1][kt][s];
-          if (m == NM) fm += kt == 0 ? Pbg[s] * g[0][s] : 0.5f * Pbg[s] * g[kt][s];
-          dq[m] = fmaf(D, fm, dq[m]);
-        }
-        dq[idT] = fmaf(D, f[3][kt][s], dq[idT]);
-      }
-      const float sc = -A.inv_dxd * (1.0f / (kt + 1));
-#pragma unroll
-      for (int m = 0; m < 5; m++) q[m][kt + 1][ii] = dq[m] * sc;
-      if (DIR == 2) {
-        q[idW][kt + 1][ii] = fmaf(sr[kt][ii], 1.0f / (kt + 1), q[idW][kt + 1][ii]);
-        if (A.bc == BC_WALL) {
-          if (kb == A.nz - 1 && ii == NG - 1) q[idW][kt + 1][ii] = 0.f;
-          if (kb == 0 && ii == 0) q[idW][kt + 1][ii] = 0.f;
-        }
-        sr[kt + 1][ii] = -q[idR][kt + 1][ii] * GRAVF;
-      }
+      for (int ii = 0; ii < NG; ii++) w = fmaf(T.wts[ii], q[idR][kt + 1].get(ii), w);
+      sa = fmaf(dtm * (-GRAVF / (kt + 2)), w, sa);
+      dtm *= A.dt;
     }
     if (kt + 1 < NA - 1) {  // products needed by the next level only
+      auto Q = [&](int m, int l) -> const V & { return l == 0 && m == idR ? rtot : (l == 0 && m == idT ? rttot : q[m][l]); };
+      // Cauchy products of the series; the not-yet-known level kt+1 of f and g enters
+      // with a zero coefficient and is left out (an IEEE multiply by zero is not
+      // removed by the compiler)
 #pragma unroll
-      for (int ii = 0; ii < NG; ii++) {
-        const float ir0 = frcp(rtot[ii]);
-        auto Q = [&](int m, int l) -> float {
-          if (l == 0) return m == idR ? rtot[ii] : (m == idT ? rttot[ii] : q[m][0][ii]);
-          return q[m][l][ii];
-        };
-        // Cauchy products of the series; the not-yet-known level kt+1 of f and g enters
-        // with a zero coefficient and is left out (an IEEE multiply by zero is not
-        // removed by the compiler)
+      for (int x = 0; x < 4; x++) {
+        V tot = q[NM][0] * Q(x + 1, kt + 1);
+        V sub = q[idR][1] * f[x][kt];
 #pragma unroll
-        for (int x = 0; x < 4; x++) {
-          float tot = 0.f;
-#pragma unroll
-          for (int ir = 0; ir <= kt + 1; ir++) {
-            tot = fmaf(Q(NM, ir), Q(x + 1, kt + 1 - ir), tot);
-            if (ir != 0) tot = fmaf(-Q(idR, ir), f[x][kt + 1 - ir][ii], tot);
-          }
-          f[x][kt + 1][ii] = tot * ir0;
+        for (int i = 1; i <= kt + 1; i++) {
+          tot = fmaT(q[NM][i], Q(x + 1, kt + 1 - i), tot);
+          if (i > 1) sub = fmaT(q[idR][i], f[x][kt + 1 - i], sub);
         }
-        // scaled (rho theta)^gamma: g~(0) = 1 + B
-        auto Gs = [&](int l) -> float { return l == 0 ? 1.f + g[0][ii] : g[l][ii]; };
-        float tg = 0.f;
-#pragma unroll
-        for (int ir = 0; ir <= kt; ir++) {
-          float term = GAMMAF * Gs(ir) * Q(idT, kt + 1 - ir);
-          if (ir != 0) term = fmaf(-Q(idT, ir), Gs(kt + 1 - ir), term);
-          tg = fmaf(kt + 1.f - ir, term, tg);
-        }
-        g[kt + 1][ii] = fmaf(tg, 1.0f / (kt + 1), GAMMAF * Gs(0) * q[idT][kt + 1][ii]) * frcp(rttot[ii]);
+        f[x][kt + 1] = (tot - sub) * ir;
       }
+      // scaled (rho theta)^gamma: g~(0) = 1 + B
+      const V one = same<NG>(1.f);
+      auto Gs = [&](int l) -> V { return l == 0 ? one + g[0] : g[l]; };
+      V tg = (2.f * GAMMAF) * (Gs(0) * q[idT][kt + 1]);  // the leading term of the sum, and outside it
+#pragma unroll
+      for (int i = 1; i <= kt; i++) {
+        const V term = GAMMAF * (g[i] * q[idT][kt + 1 - i]) - q[idT][i] * Gs(kt + 1 - i);
+        tg = fmaT((kt + 1.f - i) / (kt + 1.f), term, tg);
+      }
+      g[kt + 1] = tg * rcpT(rttot);
     }
   }
   rec.series32(q, rtot);
-  // compute_timeAvg_edges on perturbations (Spatial:2153-2177)
+  // compute_timeAvg_edges on perturbations (Spatial:2153-2177): both edges as one pair
 #pragma unroll
   for (int v = 0; v < 5; v++) {
-    float l = q[v][0][0], r = q[v][0][NG - 1];
+    F2 e = q[v][0].p[0];
     float dtmult = A.dt;
 #pragma unroll
     for (int kt = 1; kt < NA; kt++) {
-      const float c = dtmult * (1.0f / (kt + 1));
-      l = fmaf(q[v][kt][0], c, l);
-      r = fmaf(q[v][kt][NG - 1], c, r);
+      e = fmaT(dtmult * (1.0f / (kt + 1)), q[v][kt].p[0], e);
       dtmult *= A.dt;
     }
-    eL[v] = l;
-    eR[v] = r;
+    eL[v] = e.v.x;
+    eR[v] = e.v.y;
   }
-  src_avg = 0.f;
-  if (DIR == 2) {
-    float dtmult = A.dt;
-#pragma unroll
-    for (int kt = 1; kt < NA; kt++) {
-#pragma unroll
-      for (int ii = 0; ii < NG; ii++) sr[0][ii] = fmaf(sr[kt][ii], dtmult * (1.0f / (kt + 1)), sr[0][ii]);
-      dtmult *= A.dt;
-    }
-    float sa = 0.f;
-#pragma unroll
-    for (int ii = 0; ii < NG; ii++) sa = fmaf(sr[0][ii], T.wts[ii], sa);
-    src_avg = sa;
-  }
+  src_avg = sa;
 }
 
 // Upwind Riemann flux in FP32 perturbation form (Spatial:842-902, 1202-1260, 1583-1644).
@@ -509,7 +637,10 @@ struct P32 {
   static __device__ __forceinline__ void flag_timeout(const SweepArgs32 &A) {
     if (A.err) atomicOr(A.err, 1u);
   }
-  static constexpr int min_blocks(int) { return 1; }  // forcing more CTAs per SM measured slower
+  // ord 5: five CTAs of 128 threads per SM (86-93 registers): 256x256x128 step 1.160 ms,
+  // against 1.200 at the compiler's 115 (four) and 1.177 at six (80); the small-grid shapes
+  // and the x-slab sweep at four (awfl_sweep.cuh)
+  static constexpr int min_blocks(int ord) { return ord == 5 ? 5 : 1; }
   using Args = SweepArgs32;
   // rows that TMA cannot address (16-byte pitch) come by cp.async: 107 instead of about 85 us
   // for the x split of 130x100x70
@@ -552,19 +683,18 @@ struct P32 {
   static __device__ __forceinline__ void store_tend(const Args &A, long g, float x) { A.tend[g] = x; }
 };
 
-// Single-grid sweep shapes of the FP32 form, ord 5 (chunk C x lines W; measured at
-// 256x256x128 with TMA staging against x {16,8} {32,4} {4,32} {8,32} {16,16}, y {8,16}
-// {16,8} {16,16} {8,32} {4,16}, z {8,16} {16,8} {8,32} {4,64} {4,16}): x 8 x 16, y 4 x 32,
-// z 4 x 32 (y/z: a warp = 8 lines x 4 positions, 32-byte row segments).
+// Single-grid sweep shapes of the FP32 form, ord 5 (chunk C x lines W, 128 threads): x 8 x 16,
+// y 8 x 16, z 4 x 32 (y/z: a warp = 32/C lines x C positions). Measured at 256x256x128, five
+// CTAs per SM, us per split: x 8x16 374, 16x8 372, 8x8 (64 threads) 425; y 8x16 385, 4x32
+// 401, 8x8 385, 4x16 418; z 4x32 388, 8x16 408, 4x64 511, 4x16 438.
 template <> struct PolicyShape<P32, 5, 0> { static constexpr int C = 8, W = 16; };
-template <> struct PolicyShape<P32, 5, 1> { static constexpr int C = 4, W = 32; };
-
+template <> struct PolicyShape<P32, 5, 1> { static constexpr int C = 8, W = 16; };
 // The shapes for small grids (PolicyShapes, awfl_sweep.cuh).
 template <int DIR> struct PolicyShapes<P32, 5, DIR> {
   static constexpr int n = 4;
-  static constexpr int C[4] = {DIR == 0 ? 4 : 8, 16, 32, 128}, W[4] = {DIR == 0 ? 32 : 16, 8, 4, 1};
-  static constexpr double factor[4] = {DIR == 0 ? 1.0 : (DIR == 1 ? 1.05 : 1.1), DIR == 0 ? 1.15 : (DIR == 1 ? 1.2 : 1.3),
-                                       DIR == 0 ? 1.25 : (DIR == 1 ? 1.7 : 1.8), DIR == 0 ? 1.5 : 2.5};
+  static constexpr int C[4] = {DIR == 2 ? 8 : 4, 16, 32, 128}, W[4] = {DIR == 2 ? 16 : 32, 8, 4, 1};
+  static constexpr double factor[4] = {DIR == 2 ? 1.1 : 1.0, DIR == 0 ? 1.15 : (DIR == 1 ? 1.15 : 1.3),
+                                       DIR == 0 ? 1.25 : (DIR == 1 ? 1.6 : 1.8), DIR == 0 ? 1.5 : 2.5};
 };
 
 // Uploads the FP32 tables into this translation unit's constant memory.
@@ -612,6 +742,8 @@ static inline cudaError_t upload_tables32_here(int ord, const double *recon, con
     Tables32<5> t;
     fill(t, 5, 3);
     if (!structure_ok(t, 5, 3)) return cudaErrorInvalidValue;
+    for (int i = 0; i < 4; i++)  // the reconstruction's compile-time weights
+      if (fabs(idl[i] - (i == 1 ? w5::kD1 : (i == 3 ? w5::kD3 : w5::kD0))) > 1e-12 || fabs(sigma - w5::kSigma) > 1e-12) return cudaErrorInvalidValue;
     return cudaMemcpyToSymbol(c32_tab5, &t, sizeof t);
   }
   Tables32<9> t;

@@ -163,8 +163,7 @@ template <class P> struct PolicyFaceRec<P, std::void_t<decltype(P::kFaceRec)>> :
 // the neighbouring slabs (A.xh); a separate instantiation, so that the plain sweeps carry
 // none of its registers.
 // ENDS: the line's last face takes a spare lane (below): for the small-grid shapes, since
-// the large grids' sweeps, with many chunks to a line, lose more by the registers (FP32:
-// 146 instead of 126, three CTAs per SM instead of four).
+// the large grids' sweeps, with many chunks to a line, lose more by the registers.
 template <class P, int ORD, int DIR, int C, int W, bool TMA = false, bool SLAB = false, bool ENDS = false>
 __device__ __forceinline__ void sweep_tile(const typename P::Args &A, const int bx, const int by,
                                            const void *tmap = nullptr) {
@@ -660,20 +659,19 @@ __device__ __forceinline__ void sweep_tile(const typename P::Args &A, const int 
   }
 }
 
-// TMA: the policy's single-grid TMA path; its tensor map lives in the (grid-constant)
-// kernel parameter, the only place besides global memory a TMA copy may read it from.
-// CTAs per SM the register budget must allow: the policy's figure, or for the x-slab
-// sweeps of ord 5 at least AWFL_SLAB_MINB_ORD5 (4: the FP32 slab sweep drops from 142 to
-// 112 registers, no spills, and its x split of a 128x256x128 slab from 0.442 to 0.408 ms;
-// the same bound on the single-grid FP32 sweeps made them slower), and so for the
-// small-grid shapes
-#ifndef AWFL_SLAB_MINB_ORD5
-#define AWFL_SLAB_MINB_ORD5 4
+// CTAs per SM the register budget must allow: the policy's figure, or for the x-slab sweeps
+// and the small-grid shapes of ord 5 AWFL_SMALL_MINB_ORD5 (the FP32 slab sweep at 4: 142 ->
+// 107 registers and its x split of a 128x256x128 slab 0.442 -> 0.408 ms; the FP32 z split
+// of 64x64x32 at 4 / 5: 17.4 / 18.5 us)
+#ifndef AWFL_SMALL_MINB_ORD5
+#define AWFL_SMALL_MINB_ORD5 4
 #endif
 template <class P, int ORD, bool CAP> constexpr int sweep_min_blocks() {
-  return (CAP && ORD == 5 && AWFL_SLAB_MINB_ORD5 > P::min_blocks(ORD)) ? AWFL_SLAB_MINB_ORD5 : P::min_blocks(ORD);
+  return CAP && ORD == 5 ? AWFL_SMALL_MINB_ORD5 : P::min_blocks(ORD);
 }
 
+// TMA: the policy's single-grid TMA path; its tensor map lives in the (grid-constant)
+// kernel parameter, the only place besides global memory a TMA copy may read it from.
 template <class P, int ORD, int DIR, int C, int W, bool TMA, bool SLAB = false, bool ENDS = false>
 __global__ void __launch_bounds__(C *W, (sweep_min_blocks<P, ORD, SLAB || ENDS>())) sweep_kernel(const __grid_constant__ typename P::Args A) {
   if constexpr (TMA) sweep_tile<P, ORD, DIR, C, W, true, SLAB, ENDS>(A, blockIdx.x, blockIdx.y, P::tma_map(A));

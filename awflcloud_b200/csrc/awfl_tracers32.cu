@@ -54,8 +54,8 @@ struct P32Trc : P32 {
       for (int kt = 0; kt < NG - 1; kt++)
 #pragma unroll
         for (int ii = 0; ii < NG; ii++) {
-          base[(kt * NG + ii) * n + cell] = kt == 0 ? rtot[ii] : q[idR][kt][ii];
-          base[(NS + kt * NG + ii) * n + cell] = q[nm][kt][ii];
+          base[(kt * NG + ii) * n + cell] = kt == 0 ? rtot.get(ii) : q[idR][kt].get(ii);
+          base[(NS + kt * NG + ii) * n + cell] = q[nm][kt].get(ii);
         }
     }
   };
