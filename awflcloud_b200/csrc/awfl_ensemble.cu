@@ -108,6 +108,40 @@ void tiles(const awfl_config &c, int dir, int W, int *nbx, int *nby) {
   else { *nbx = (c.nx + W - 1) / W; *nby = c.ny; }
 }
 
+// The shape an untuned ensemble starts with: the cheapest of the candidates by the sweeps' cost
+// model (awfl_sweep.cuh) over the members' tiles, spread over the SMs and at least as long
+// as the longest line, times what the shape costs on a full chip (measured, 24 members of
+// 32..96 cells a side: FP32 us per launch x 327 343 237 262, y 239 242 228 237, z 262 294
+// 243 284 in the candidates' order; FP64 x 865 1054 741 766, y 774 757 844 822, z 875 890 931
+// 1000). That ensemble: FP32 1.63 -> 1.40 ms for two steps, FP64 4.99 -> 4.72; 4 members of
+// 16..40: FP32 0.114 -> 0.099.
+int default_shape(const awfl_ensemble *e, int dir) {
+  static const double f32[3][4] = {{1.38, 1.45, 1.0, 1.1}, {1.05, 1.06, 1.0, 1.04}, {1.08, 1.2, 1.0, 1.17}};
+  static const double f64[3][4] = {{1.17, 1.42, 1.0, 1.03}, {1.02, 1.0, 1.11, 1.09}, {1.0, 1.02, 1.07, 1.15}};
+  if (e->ord != 5) return 0;
+  int best = 0;
+  double cost = 0;
+  for (int s = 0; s < ens_num_shapes(e->ord, dir); s++) {
+    int C, W;
+    ens_shape(e->ord, dir, s, &C, &W);
+    double units = 0, longest = 0, ctas = 0;  // in CTAs of 128 threads
+    for (awfl_ctx *m : e->mem) {
+      if (dir == 1 && ctx_sim2d(m)) continue;
+      int nbx, nby;
+      tiles(ctx_cfg(m), dir, W, &nbx, &nby);
+      const double chunks = (line_len(ctx_cfg(m), dir) + C - 1) / C + 0.35, n = (double)nbx * nby * (C * W / 128.0);
+      units += n * chunks;
+      ctas += n;
+      longest = std::max(longest, chunks);
+    }
+    const double k = std::min(4.0, std::ceil(ctas / e->nsm));  // resident per SM
+    const double c = (e->prec == AWFL_FP32 ? f32 : f64)[dir][s] * (0.6 + 0.4 * k) *
+                     std::max(longest, k > 0 ? units / (k * e->nsm) : 0.0);
+    if (s == 0 || c < cost) { best = s; cost = c; }
+  }
+  return best;
+}
+
 // Builds the three work lists for the current shapes and the given states (the bound
 // ones, or the tuner's scratch copies) into one device allocation.
 int build_lists(awfl_ensemble *e, const std::vector<void *> &states, void **d_out, EnsList<SweepArgs> (&l64)[3],
@@ -277,7 +311,10 @@ int awfl_ensemble_create(const awfl_config *cfgs, int nmembers, int device, awfl
   e->state.assign(nmembers, nullptr);
   e->dt.assign(nmembers, 0.0);
   e->nsm = ctx_nsm(e->mem[0]);
-  for (int dir = 0; dir < 3; dir++) e->tune_ms[dir].assign(ens_num_shapes(e->ord, dir), -1.f);
+  for (int dir = 0; dir < 3; dir++) {
+    e->tune_ms[dir].assign(ens_num_shapes(e->ord, dir), -1.f);
+    e->shape[dir] = default_shape(e, dir);
+  }
   *out = e;
   return AWFL_OK;
 }
