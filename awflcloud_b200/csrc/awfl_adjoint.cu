@@ -90,7 +90,7 @@ struct P64Rec : P64 {
   }
 };
 template <int ORD, int DIR> struct PolicyShape<P64Rec, ORD, DIR> : PolicyShape<P64, ORD, DIR> {};
-template <int ORD, int DIR> struct PolicyShapes<P64Rec, ORD, DIR> : SmallShapes<ORD, DIR> {};
+template <int ORD, int DIR> struct PolicyShapes<P64Rec, ORD, DIR> : RecordShapes<ORD, DIR> {};
 
 cudaError_t launch_sweep_rec(int ord, int dir, const SweepArgs &A, cudaStream_t st) {
   return launch_sweep_any<P64Rec>(ord, dir, A, st);

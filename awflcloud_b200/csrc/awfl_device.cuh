@@ -318,33 +318,38 @@ __device__ __forceinline__ double add_divk(const double &x, const double &y, int
   return x + divk(y, k);
 }
 
+// sum_s deriv(s, ii) x[s] on doubles, but for the sign of a zero sum: without the leading
+// 0 +, and at ord 5, whose matrix is {-3 4 -1; -1 0 1; 1 -4 3}, the products by 0 and +-1; a
+// product by 4 is exact and goes into an FMA.
+template <int ORD> __device__ __forceinline__ double deriv_sum(const double (&x)[OrdTraits<ORD>::NGLL], int ii) {
+  if constexpr (ORD == 5) {
+    if (ii == 0) return __fma_rn(4., x[1], -3. * x[0]) - x[2];
+    if (ii == 1) return x[2] - x[0];
+    return __fma_rn(-4., x[1], x[0]) + 3. * x[2];
+  } else {
+    const Tables<ORD> &T = tab<ORD>();
+    double d = T.deriv[ii] * x[0];
+#pragma unroll
+    for (int s = 1; s < OrdTraits<ORD>::NGLL; s++) d += T.deriv[s * OrdTraits<ORD>::NGLL + ii] * x[s];
+    return d;
+  }
+}
+
 // -(sum_s deriv(s, ii) x[s]) / dx / k: level k of a variable's time series from its flux x at
-// level k-1. On doubles the sum leaves out what changes at most the sign of a zero level
-// (which ends in sums that do not see it: the edge states start from level 0, never -0): the
-// leading 0 +, and at ord 5, whose matrix is {-3 4 -1; -1 0 1; 1 -4 3}, the products by 0
-// and +-1; a product by 4 is exact and goes into an FMA. The quotient is div_known's, a
-// power-of-two k folded into the divisor's pair.
+// level k-1. The sign of a zero level ends in sums that do not see it (the edge states start
+// from level 0, never -0). On doubles the quotient is div_known's, a power-of-two k folded
+// into the divisor's pair.
 template <int ORD, class Sc>
 __device__ __forceinline__ Sc deriv_term(const Sc (&x)[OrdTraits<ORD>::NGLL], int ii, int k, const SweepArgs &A) {
-  constexpr int NG = OrdTraits<ORD>::NGLL;
-  const Tables<ORD> &T = tab<ORD>();
   if constexpr (std::is_same<Sc, double>::value) {
-    double d;
-    if constexpr (ORD == 5) {
-      if (ii == 0) d = __fma_rn(4., x[1], -3. * x[0]) - x[2];
-      else if (ii == 1) d = x[2] - x[0];
-      else d = __fma_rn(-4., x[1], x[0]) + 3. * x[2];
-    } else {
-      d = T.deriv[ii] * x[0];
-#pragma unroll
-      for (int s = 1; s < NG; s++) d += T.deriv[s * NG + ii] * x[s];
-    }
+    const double d = deriv_sum<ORD>(x, ii);
     if ((k & (k - 1)) == 0) return div_known(d, A.nrdx_h * (1.0 / k), A.nrdx_l * (1.0 / k));
     return divk(div_known(d, A.nrdx_h, A.nrdx_l), k);
   } else {
+    constexpr int NG = OrdTraits<ORD>::NGLL;
     Sc d = 0.;
 #pragma unroll
-    for (int s = 0; s < NG; s++) d += T.deriv[s * NG + ii] * x[s];
+    for (int s = 0; s < NG; s++) d += tab<ORD>().deriv[s * NG + ii] * x[s];
     return divk(divd(-d, rcp_known(A.dxd, A.rdxd)), k);
   }
 }

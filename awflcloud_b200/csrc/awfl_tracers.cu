@@ -98,7 +98,7 @@ struct P64Trc : P64 {
 };
 
 template <int ORD, int DIR> struct PolicyShape<P64Trc, ORD, DIR> : PolicyShape<P64, ORD, DIR> {};
-template <int ORD, int DIR> struct PolicyShapes<P64Trc, ORD, DIR> : SmallShapes<ORD, DIR> {};
+template <int ORD, int DIR> struct PolicyShapes<P64Trc, ORD, DIR> : RecordShapes<ORD, DIR> {};
 
 namespace {
 
@@ -124,14 +124,14 @@ __device__ __forceinline__ double trc_divisor(const TracerArgs &T, int hs, int k
 __device__ __forceinline__ double trc_dens(const TracerArgs &T, int hs, int k) { return T.A.dens_c[hs + k]; }
 // a / (the upwind density of face fi), correctly rounded through its recorded reciprocal
 __device__ __forceinline__ double trc_div_up(const TracerArgs &T, double a, long fi) {
-  return divr_any(a, rcp_known(T.RUP[fi], T.YUP[fi]));
+  return divp_any(a, rcp_known(T.RUP[fi], T.YUP[fi]));
 }
 // factor and scaled flux of one face from its upwind cell's two faces (f1 = min(., 0) of
 // the left one, f2 = max(., 0) of the right one; q: the cell's tracer / density)
 __device__ __forceinline__ double limit_face(const TracerArgs &T, double F, double f1, double f2, double q,
                                              double dens) {
   const double eps = 1.e-10;
-  const double fluxOut = divr_any(T.A.dt * (f2 - f1), rcp_known(T.A.dxd, T.A.rdxd));
+  const double fluxOut = divp_any(T.A.dt * (f2 - f1), rcp_known(T.A.dxd, T.A.rdxd));
   const double r = q * dens / (fluxOut + eps);
   return F * (1. < r ? 1. : r);  // F * min(1, r)
 }
@@ -205,86 +205,77 @@ __global__ void __launch_bounds__(128, ORD == 5 ? AWFL_TRC_CELL_MINB : 1) tracer
       s[m] = tr[(p - p0) * gsd];
     }
   }
-  double rt[NG][NG], rut[NG][NG];
-  // a stencil of zeros (a tracer absent from this part of the domain) reconstructs to +0
-  // at every GLL point, WENO or not: every sum of the reconstruction starts at +0 and adds
-  // products with a zero factor, and its weights stay finite (eps keeps them off 1/0)
+  // A stencil of zeros (a tracer absent from this part of the domain) reconstructs to +0 at
+  // every GLL point, WENO or not (every sum of the reconstruction starts at +0 and adds
+  // products with a zero factor, and its weights stay finite: eps keeps them off 1/0); its
+  // series is zeros, whose signs the edges' sums from +0 do not keep: both edges are +0.
   bool zero = true;
 #pragma unroll
   for (int m = 0; m < ORD; m++) zero = zero && s[m] == 0.;
-  if (zero) {
-#pragma unroll
-    for (int ii = 0; ii < NG; ii++) rt[0][ii] = 0.;
-  } else {
+  double tl = 0., trr = 0.;
+  if (!zero) {
+    double rt[NG][NG], rut[NG][NG];
     reconstruct_gll_any<ORD>(s, rt[0], A.weno_s != 0);
-  }
-  double rser[NG - 1][NG], ruser[NG - 1][NG];
-  {
-    const double *r = T.R + c, *u = T.U + c;  // plane by plane, ncell apart
+    double rser[NG - 1][NG], ruser[NG - 1][NG];
+    {
+      const double *r = T.R + c, *u = T.U + c;  // plane by plane, ncell apart
 #pragma unroll
-    for (int kt = 0; kt < NG - 1; kt++)
+      for (int kt = 0; kt < NG - 1; kt++)
 #pragma unroll
-      for (int ii = 0; ii < NG; ii++) {
-        rser[kt][ii] = *r;
-        ruser[kt][ii] = *u;
-        r += ncell;
-        u += ncell;
-      }
-  }
-  // the divisors through their correctly rounded reciprocals (IEEE quotients bit for bit):
-  // the GLL points' densities (reciprocals recorded by the sweep) and dx
-  Rcp<double> rr[NG];
-  {
-    const double *y = T.Y + c;
+        for (int ii = 0; ii < NG; ii++) {
+          rser[kt][ii] = *r;
+          ruser[kt][ii] = *u;
+          r += ncell;
+          u += ncell;
+        }
+    }
+    // the divisors through their correctly rounded reciprocals (IEEE quotients bit for bit):
+    // the GLL points' densities (reciprocals recorded by the sweep) and dx
+    Rcp<double> rr[NG];
+    {
+      const double *y = T.Y + c;
 #pragma unroll
-    for (int ii = 0; ii < NG; ii++) rr[ii] = rcp_known(rser[0][ii], y[ii * (long)ncell]);
-  }
-  const Rcp<double> rdx = rcp_known(A.dxd, A.rdxd);
-  const Tables<ORD> &TB = tab<ORD>();
-#pragma unroll
-  for (int ii = 0; ii < NG; ii++) {
-    rt[0][ii] *= rser[0][ii];
-    if (posdef) rt[0][ii] = dmax(0., rt[0][ii]);
-  }
-#pragma unroll
-  for (int ii = 0; ii < NG; ii++) rut[0][ii] = divr_any(rt[0][ii] * ruser[0][ii], rr[ii]);
-  // diffTransformTracer (Spatial:2095-2125)
-#pragma unroll
-  for (int kt = 1; kt < NG; kt++)
-#pragma unroll
-    for (int ii = 0; ii < NG; ii++) rut[kt][ii] = 0;
-#pragma unroll
-  for (int kt = 0; kt < NG - 1; kt++) {
+      for (int ii = 0; ii < NG; ii++) rr[ii] = rcp_known(rser[0][ii], y[ii * (long)ncell]);
+    }
 #pragma unroll
     for (int ii = 0; ii < NG; ii++) {
-      double df = 0;
-#pragma unroll
-      for (int q = 0; q < NG; q++) df += TB.deriv[q * NG + ii] * rut[kt][q];
-      rt[kt + 1][ii] = divk_any(divr_any(-df, rdx), kt + 1);
+      rt[0][ii] *= rser[0][ii];
+      if (posdef) rt[0][ii] = dmax(0., rt[0][ii]);
     }
-    if (kt + 1 < NG - 1) {  // the last level of rho*u*tracer reaches no edge
 #pragma unroll
-      for (int ii = 0; ii < NG; ii++) {
-        double tot = 0;
+    for (int ii = 0; ii < NG; ii++) rut[0][ii] = divp_any(rt[0][ii] * ruser[0][ii], rr[ii]);
+    // diffTransformTracer (Spatial:2095-2125); level kt+1 of rut is still zero where the
+    // reference's product reads it: that term is left out
 #pragma unroll
-        for (int ir = 0; ir <= kt + 1; ir++)
-          tot += ruser[ir][ii] * rt[kt + 1 - ir][ii] - rser[ir][ii] * rut[kt + 1 - ir][ii];
-        rut[kt + 1][ii] = divr_any(tot, rr[ii]);
+    for (int kt = 0; kt < NG - 1; kt++) {
+#pragma unroll
+      for (int ii = 0; ii < NG; ii++)
+        rt[kt + 1][ii] = divk_any(div_known_any(deriv_sum<ORD>(rut[kt], ii), -A.dxd, A.nrdx_h, A.nrdx_l), kt + 1);
+      if (kt + 1 < NG - 1) {  // the last level of rho*u*tracer reaches no edge
+#pragma unroll
+        for (int ii = 0; ii < NG; ii++) {
+          double tot = ruser[0][ii] * rt[kt + 1][ii];
+#pragma unroll
+          for (int ir = 1; ir <= kt + 1; ir++)
+            tot += ruser[ir][ii] * rt[kt + 1 - ir][ii] - rser[ir][ii] * rut[kt + 1 - ir][ii];
+          rut[kt + 1][ii] = divp_any(tot, rr[ii]);
+        }
       }
     }
-  }
-  // compute_timeAvg_edges (Spatial:2153-2177), then the positivity clamp of the edges
-  double tl = rt[0][0], trr = rt[0][NG - 1];
-  double dtmult = A.dt;
+    // compute_timeAvg_edges (Spatial:2153-2177), then the positivity clamp of the edges
+    tl = rt[0][0];
+    trr = rt[0][NG - 1];
+    double dtmult = A.dt;
 #pragma unroll
-  for (int kt = 1; kt < NG; kt++) {
-    tl += divk_any(rt[kt][0] * dtmult, kt + 1);
-    trr += divk_any(rt[kt][NG - 1] * dtmult, kt + 1);
-    dtmult *= A.dt;
-  }
-  if (posdef) {
-    tl = dmax(0., tl);
-    trr = dmax(0., trr);
+    for (int kt = 1; kt < NG; kt++) {
+      tl += divk_any(rt[kt][0] * dtmult, kt + 1);
+      trr += divk_any(rt[kt][NG - 1] * dtmult, kt + 1);
+      dtmult *= A.dt;
+    }
+    if (posdef) {
+      tl = dmax(0., tl);
+      trr = dmax(0., trr);
+    }
   }
   // the fluxes of the faces this cell is upwind of
   const long fs = DIR == 0 ? 1 : (DIR == 1 ? G.nx : (long)G.nx * G.ny), fl = G.face(k, j, i);
