@@ -40,7 +40,7 @@ struct awfl_ctx {
   double *d_dens_c = nullptr, *d_denstheta_c = nullptr, *d_dens_g = nullptr, *d_denstheta_g = nullptr,
          *d_pres_g = nullptr;
   double *d_pres_c = nullptr;           // hydrostatic pressure cell averages (output)
-  unsigned long long *d_cfl = nullptr;  // CFL reduction result (8 bytes)
+  unsigned long long *d_cfl = nullptr;  // CFL reduction: 3 maxima, a block counter, 3 results
   unsigned int *d_err = nullptr;        // a sweep's bounded wait gave up (the next 8 bytes)
   // FP32 form: FP32 copies of FP64 background constants (awfl_fp32_args.h)
   float *d_bg32 = nullptr;
@@ -499,7 +499,7 @@ int awfl_create(const awfl_config *cfg, int device, awfl_ctx **out) {
   c->d_pres_g = c->d_denstheta_g + nz * g;
   c->d_pres_c = c->d_pres_g + nz * g;
   c->d_cfl = reinterpret_cast<unsigned long long *>(c->d_pres_c + (nz + 2 * hs));
-  c->d_err = reinterpret_cast<unsigned int *>(c->d_cfl + 1);
+  c->d_err = reinterpret_cast<unsigned int *>(c->d_cfl + 7);
   std::vector<double> h;
   h.reserve(nbg);
   h.insert(h.end(), c->dens_c.begin(), c->dens_c.end());
@@ -509,7 +509,7 @@ int awfl_create(const awfl_config *cfg, int device, awfl_ctx **out) {
   h.insert(h.end(), c->pres_g.begin(), c->pres_g.end());
   h.insert(h.end(), c->pres_c.begin(), c->pres_c.end());
   e = cudaMemcpy(c->d_bg, h.data(), nbg * sizeof(double), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemset(c->d_err, 0, sizeof(unsigned int));
+  if (e == cudaSuccess) e = cudaMemset(c->d_cfl, 0, 7 * sizeof(unsigned long long) + sizeof(unsigned int));  // and d_err
   if (e != cudaSuccess) { cuda_fail(nullptr, e, "upload background"); g_create_error = "upload background: " + std::string(cudaGetErrorString(e)); cudaFree(c->d_bg); delete c; return AWFL_ERR_CUDA; }
   if (cfg->precision == AWFL_FP32) {
     rc = build_bg32(c);
@@ -740,22 +740,19 @@ int awfl_cfl(awfl_ctx *c, const void *d_state, double cfl, double *h_dt, void *s
   int rc = set_device(c);
   if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
-  static const unsigned long long inf_bits = 0x7ff0000000000000ULL;
-  cudaError_t e = cudaMemcpyAsync(c->d_cfl, &inf_bits, sizeof inf_bits, cudaMemcpyHostToDevice, st);
-  if (e != cudaSuccess) return cuda_fail(c, e, "awfl_cfl init");
-  if (fp32(c))
-    e = launch_cfl_fp32((const float *)d_state, c->d_dens_c, c->d_denstheta_c, cfl, c->dx, c->dy, c->dz, c->cfg.nx,
-                        c->cfg.ny, c->cfg.nz, c->hs, c->nsm, c->d_cfl, st);
-  else
-    e = launch_cfl_fp64((const double *)d_state, c->d_dens_c, c->d_denstheta_c, cfl, c->dx, c->dy, c->dz, c->cfg.nx,
-                        c->cfg.ny, c->cfg.nz, c->hs, c->nsm, c->d_cfl, st);
+  double *result = reinterpret_cast<double *>(c->d_cfl + 4), speed[3];
+  cudaError_t e = launch_cfl(d_state, fp32(c), c->d_dens_c, c->d_denstheta_c, c->cfg.nx, c->cfg.ny, c->cfg.nz, c->hs,
+                             c->nsm, c->d_cfl, result, st);
   if (e != cudaSuccess) return cuda_fail(c, e, "cfl kernel");
-  unsigned long long bits = 0;
-  e = cudaMemcpyAsync(&bits, c->d_cfl, sizeof bits, cudaMemcpyDeviceToHost, st);
+  e = cudaMemcpyAsync(speed, result, sizeof speed, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return cuda_fail(c, e, "awfl_cfl readback");
-  double dt;
-  std::memcpy(&dt, &bits, sizeof dt);
+  const double dx[3] = {c->dx, c->dy, c->dz};
+  double dt = INFINITY;
+  for (int d = 0; d < 3; d++) {
+    const double t = cfl * dx[d] / speed[d];
+    dt = t < dt ? t : dt;
+  }
   if (!(dt > 0) || !std::isfinite(dt)) return fail(c, AWFL_ERR_STATE, "awfl_cfl: non-finite or non-positive time step (%g)", dt);
   *h_dt = dt;
   return AWFL_OK;

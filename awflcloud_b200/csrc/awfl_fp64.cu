@@ -7,6 +7,7 @@
 //                          (Spatial:631-957 x, 994-1310 y, 1351-1696 z; Temporal_ader.h:63-65)
 //   apply_kernel           K6 apply alone (Temporal_ader.h:63-65)
 //   add_zero_kernel        the apply of a sim2d y split's zero tendencies
+//   apply32_kernel         the FP32 form's compensated apply
 //   cfl_kernel             K0 CFL time step (Spatial:169-183)
 //   init_state_kernel      K9 initial data quadrature (Spatial:428-485)
 #include <cuda_runtime.h>
@@ -25,113 +26,163 @@ cudaError_t launch_sweep_fp64(int ord, int dir, const SweepArgs &A, cudaStream_t
 
 
 // ------------------------------------------------------------------------------------
-// K6 apply (Temporal_ader.h:63-65): state(l,hs+k,hs+j,hs+i) += dt * tend(l,k,j,i).
+// K6 apply (Temporal_ader.h:63-65): state(l,hs+k,hs+j,hs+i) += dt * tend(l,k,j,i). A thread
+// takes one cell's five variables: one index division per cell, ten loads in flight. Bound by
+// its bytes (120 per cell); 256x256x128: 308 -> 171 us, 0.91 of the
+// measured copy bandwidth; 130x100x70: 31.5 -> 14.7.
 // ------------------------------------------------------------------------------------
-__global__ void apply_kernel(double *state, const double *tend, double dt, int nx, int ny, int nz, int hs) {
-  const long n = 5L * nz * ny * nx;
-  for (long idx = blockIdx.x * (long)blockDim.x + threadIdx.x; idx < n; idx += (long)gridDim.x * blockDim.x) {
-    long r = idx;
-    const int i = r % nx; r /= nx;
-    const int j = r % ny; r /= ny;
-    const int k = r % nz; r /= nz;
-    const int l = (int)r;
-    const long s = (((long)l * (nz + 2 * hs) + hs + k) * (ny + 2 * hs) + hs + j) * (nx + 2 * hs) + hs + i;
-    state[s] += dt * tend[idx];
+constexpr int kCellThreads = 256;
+// threads over the cells of a plane (x), planes (y)
+dim3 cell_grid(int nx, int ny, int nz) {
+  return dim3((unsigned)(((long)nx * ny + kCellThreads - 1) / kCellThreads), (unsigned)nz);
+}
+struct CellAt {
+  long s, c;  // halo-inclusive and interior offset of the cell in variable 0
+  bool in;
+  __device__ __forceinline__ CellAt(int nx, int ny, int hs) {
+    const long q = blockIdx.x * (long)kCellThreads + threadIdx.x;
+    const int k = blockIdx.y;
+    in = q < (long)nx * ny;
+    const long j = q < (1L << 31) ? (long)((unsigned)q / (unsigned)nx) : q / nx;
+    c = (long)k * nx * ny + q;
+    s = ((hs + k) * (long)(ny + 2 * hs) + hs + j) * (nx + 2 * hs) + hs + (q - j * nx);
   }
+};
+
+__global__ void __launch_bounds__(kCellThreads) apply_kernel(double *state, const double *tend, double dt, int nx, int ny, int nz, int hs) {
+  const CellAt p(nx, ny, hs);
+  if (!p.in) return;
+  const long n = (long)nz * ny * nx, sv = (long)(nz + 2 * hs) * (ny + 2 * hs) * (nx + 2 * hs);
+#pragma unroll
+  for (int l = 0; l < 5; l++) state[p.s + l * sv] += dt * tend[p.c + l * n];
 }
 
 cudaError_t launch_apply_fp64(double *state, const double *tend, double dt, int nx, int ny, int nz, int hs,
                               int nsm, cudaStream_t st) {
-  const long n = 5L * nz * ny * nx;
-  long blocks = (n + 255) / 256;
-  const long cap = (long)nsm * 8;
-  if (blocks > cap) blocks = cap;
-  if (blocks < 1) blocks = 1;
-  apply_kernel<<<(unsigned)blocks, 256, 0, st>>>(state, tend, dt, nx, ny, nz, hs);
+  (void)nsm;
+  apply_kernel<<<cell_grid(nx, ny, nz), kCellThreads, 0, st>>>(state, tend, dt, nx, ny, nz, hs);
+  return cudaGetLastError();
+}
+
+// The same with the Kahan-compensated update of an FP32 state (P32::apply).
+__global__ void __launch_bounds__(kCellThreads) apply32_kernel(float *state, float *comp, const float *tend, float dt, int nx, int ny, int nz, int hs) {
+  const CellAt p(nx, ny, hs);
+  if (!p.in) return;
+  const long n = (long)nz * ny * nx, sv = (long)(nz + 2 * hs) * (ny + 2 * hs) * (nx + 2 * hs);
+#pragma unroll
+  for (int l = 0; l < 5; l++) {
+    const long s = p.s + l * sv;
+    const float old = state[s], y = __fmaf_rn(dt, tend[p.c + l * n], -comp[s]), t = __fadd_rn(old, y);
+    comp[s] = __fsub_rn(__fsub_rn(t, old), y);
+    state[s] = t;
+  }
+}
+
+cudaError_t launch_apply_fp32(float *state, float *comp, const float *tend, float dt, int nx, int ny, int nz, int hs,
+                              int nsm, cudaStream_t st) {
+  (void)nsm;
+  apply32_kernel<<<cell_grid(nx, ny, nz), kCellThreads, 0, st>>>(state, comp, tend, dt, nx, ny, nz, hs);
   return cudaGetLastError();
 }
 
 // x += dt*0 on the interior of nplanes planes of the state layout: what the apply
 // (Temporal_ader.h:63-69) does with the zero tendencies of a sim2d y split (Spatial:572-575).
 // It changes no value; a -0 becomes +0, as in the reference.
-__global__ void add_zero_kernel(double *p, int nplanes, int nx, int ny, int nz, int hs) {
-  const long n = (long)nplanes * nz * ny * nx;
-  for (long idx = blockIdx.x * (long)blockDim.x + threadIdx.x; idx < n; idx += (long)gridDim.x * blockDim.x) {
-    long r = idx;
-    const int i = r % nx; r /= nx;
-    const int j = r % ny; r /= ny;
-    const int k = r % nz; r /= nz;
-    const int l = (int)r;
-    const long s = (((long)l * (nz + 2 * hs) + hs + k) * (ny + 2 * hs) + hs + j) * (nx + 2 * hs) + hs + i;
-    p[s] = __dadd_rn(p[s], 0.0);
-  }
+__global__ void __launch_bounds__(kCellThreads) add_zero_kernel(double *x, int nplanes, int nx, int ny, int nz, int hs) {
+  const CellAt p(nx, ny, hs);
+  if (!p.in) return;
+  const long sv = (long)(nz + 2 * hs) * (ny + 2 * hs) * (nx + 2 * hs);
+  for (int l = 0; l < nplanes; l++) x[p.s + l * sv] = __dadd_rn(x[p.s + l * sv], 0.0);
 }
 
 cudaError_t launch_add_zero_fp64(double *p, int nplanes, int nx, int ny, int nz, int hs, int nsm, cudaStream_t st) {
-  const long n = (long)nplanes * nz * ny * nx;
-  long blocks = (n + 255) / 256;
-  const long cap = (long)nsm * 8;
-  if (blocks > cap) blocks = cap;
-  if (blocks < 1) blocks = 1;
-  add_zero_kernel<<<(unsigned)blocks, 256, 0, st>>>(p, nplanes, nx, ny, nz, hs);
+  (void)nsm;
+  add_zero_kernel<<<cell_grid(nx, ny, nz), kCellThreads, 0, st>>>(p, nplanes, nx, ny, nz, hs);
   return cudaGetLastError();
 }
 
 // ------------------------------------------------------------------------------------
-// K0 CFL (Spatial:169-183): per-cell min(cfl*dx/max|u+-cs|, ...); block min in shared
-// memory, then an atomic min on the bit pattern (valid for non-negative doubles) into
-// *out, which the caller initialises to +inf.
+// K0 CFL (Spatial:169-183), FP64 from either state form. The step is the minimum over cells
+// and directions of RN(cfl*dx / m), m = max|u +- cs|: division is monotone under rounding, so
+// that is RN(cfl*dx / max m), and the kernel only reduces the three largest speeds; the host
+// divides. The blocks' maxima meet in acc[0..2] (bit patterns of non-negative doubles), and
+// the last block (counted in acc[3]) moves them to `result` and zeroes acc for the next call.
+// What a NaN speed hides is what the reference's comparisons hide: of the cell's directions,
+// those before it in the order x, y, z. A cell's five quotients share its density's
+// reciprocal; a cell with a speed that is not finite is evaluated again with plain divisions,
+// whose infinities and NaN differ. Few blocks walk over the planes, so that few atomics
+// follow. awfl_cfl with its read-back, 256x256x128: 216 -> 138 us; 130x100x70: 54 -> 42.
 // ------------------------------------------------------------------------------------
-__global__ void cfl_kernel(const double *state, const double *dens_c, const double *denstheta_c,
-                           double cfl, double dx, double dy, double dz, int nx, int ny, int nz, int hs,
-                           unsigned long long *out) {
-  __shared__ double red[256];
-  double best = __longlong_as_double(0x7ff0000000000000LL);  // +inf
-  const long n = (long)nz * ny * nx;
-  const long sy = nx + 2 * hs, sz = (long)(ny + 2 * hs) * sy, sv = (long)(nz + 2 * hs) * sz;
-  for (long idx = blockIdx.x * (long)blockDim.x + threadIdx.x; idx < n; idx += (long)gridDim.x * blockDim.x) {
-    const int i = idx % nx;
-    const int j = (idx / nx) % ny;
-    const int k = idx / ((long)nx * ny);
-    const long s = (hs + k) * sz + (hs + j) * sy + hs + i;
-    const double r = state[s] + dens_c[hs + k];
-    const double u = state[s + sv] / r;
-    const double v = state[s + 2 * sv] / r;
-    const double w = state[s + 3 * sv] / r;
-    const double t = (state[s + 4 * sv] + denstheta_c[hs + k]) / r;
-    const double p = C0 * pow_cr(r * t, GAMMA);
-    const double cs = sqrt(GAMMA * p / r);
-    const double au = fabs(u - cs), bu = fabs(u + cs);
-    const double av = fabs(v - cs), bv = fabs(v + cs);
-    const double aw = fabs(w - cs), bw = fabs(w + cs);
-    const double udt = cfl * dx / (au > bu ? au : bu);
-    const double vdt = cfl * dy / (av > bv ? av : bv);
-    const double wdt = cfl * dz / (aw > bw ? aw : bw);
-    const double m1 = udt < vdt ? udt : vdt;
-    const double d = m1 < wdt ? m1 : wdt;
-    best = d < best ? d : best;
+template <bool PLAIN>
+__device__ __forceinline__ void cell_speeds(double r, const double (&m)[3], double rt, double (&out)[3]) {
+  const Rcp<double> y = PLAIN ? rcp_known(r, 0.) : make_rcp<double>(r);
+  auto over = [&](double a) { return PLAIN ? a / r : divp(a, y); };
+  const double t = over(rt);
+  const double cs = sqrt(over(GAMMA * (C0 * (PLAIN ? pow_cr(r * t, GAMMA) : pow_gamma_cr(r * t)))));
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    const double u = over(m[d]), a = fabs(u - cs), b = fabs(u + cs);
+    out[d] = a > b ? a : b;
   }
-  red[threadIdx.x] = best;
-  __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) {
-      const double o = red[threadIdx.x + s];
-      if (o < red[threadIdx.x]) red[threadIdx.x] = o;
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) atomicMin(out, (unsigned long long)__double_as_longlong(red[0]));
+}
+static __device__ __noinline__ void cell_speeds_plain(double r, double m0, double m1, double m2, double rt, double *out) {
+  const double m[3] = {m0, m1, m2};
+  double o[3];
+  cell_speeds<true>(r, m, rt, o);
+  for (int d = 0; d < 3; d++) out[d] = o[d];
 }
 
-cudaError_t launch_cfl_fp64(const double *state, const double *dens_c, const double *denstheta_c, double cfl,
-                            double dx, double dy, double dz, int nx, int ny, int nz, int hs, int nsm,
-                            unsigned long long *d_out, cudaStream_t st) {
-  const long n = (long)nz * ny * nx;
-  long blocks = (n + 255) / 256;
-  const long cap = (long)nsm * 8;
-  if (blocks > cap) blocks = cap;
-  if (blocks < 1) blocks = 1;
-  cfl_kernel<<<(unsigned)blocks, 256, 0, st>>>(state, dens_c, denstheta_c, cfl, dx, dy, dz, nx, ny, nz, hs, d_out);
+template <class T>
+__global__ void __launch_bounds__(kCellThreads) cfl_kernel(const T *state, const double *dens_c, const double *denstheta_c, int nx, int ny,
+                                                           int nz, int hs, unsigned long long *acc, double *result) {
+  const long plane = (long)nx * ny;
+  const long sy = nx + 2 * hs, sz = (long)(ny + 2 * hs) * sy, sv = (long)(nz + 2 * hs) * sz;
+  double best[3] = {0., 0., 0.};
+  for (long q = blockIdx.x * (long)kCellThreads + threadIdx.x; q < plane; q += (long)gridDim.x * kCellThreads) {
+    const long j = q < (1L << 31) ? (long)((unsigned)q / (unsigned)nx) : q / nx;
+    const T *p = state + (hs + blockIdx.y) * sz + (hs + j) * sy + hs + (q - j * nx);
+    for (int k = blockIdx.y; k < nz; k += gridDim.y, p += gridDim.y * sz) {
+      const double r = (double)p[0] + dens_c[hs + k], rt = (double)p[4 * sv] + denstheta_c[hs + k];
+      const double m[3] = {(double)p[sv], (double)p[2 * sv], (double)p[3 * sv]};
+      double v[3];
+      cell_speeds<false>(r, m, rt, v);
+      if (!(v[0] + v[1] + v[2] < 1e300)) cell_speeds_plain(r, m[0], m[1], m[2], rt, v);
+      if (v[2] == v[2]) {
+        if (v[1] == v[1] && v[0] > best[0]) best[0] = v[0];
+        if (v[1] > best[1]) best[1] = v[1];
+        if (v[2] > best[2]) best[2] = v[2];
+      }
+    }
+  }
+  __shared__ double red[3][kCellThreads / 32];
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) best[d] = fmax(best[d], __shfl_xor_sync(0xffffffffu, best[d], s));
+    if (threadIdx.x % 32 == 0) red[d][threadIdx.x / 32] = best[d];
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      double m = red[d][0];
+      for (int w = 1; w < kCellThreads / 32; w++) m = fmax(m, red[d][w]);
+      atomicMax(acc + d, (unsigned long long)__double_as_longlong(m));
+    }
+    __threadfence();
+    if (atomicAdd(acc + 3, 1ULL) == (unsigned long long)gridDim.x * gridDim.y - 1) {  // the last block
+      for (int d = 0; d < 3; d++) result[d] = __longlong_as_double((long long)atomicExch(acc + d, 0ULL));
+      acc[3] = 0;
+    }
+  }
+}
+
+cudaError_t launch_cfl(const void *state, int fp32, const double *dens_c, const double *denstheta_c, int nx, int ny,
+                       int nz, int hs, int nsm, unsigned long long *acc, double *result, cudaStream_t st) {
+  const long bx = ((long)nx * ny + kCellThreads - 1) / kCellThreads, most = (long)nsm * 8;
+  const dim3 grid((unsigned)(bx < most ? bx : most), (unsigned)(bx >= most ? 1 : (most / bx < nz ? most / bx : nz)));
+  if (fp32) cfl_kernel<float><<<grid, kCellThreads, 0, st>>>((const float *)state, dens_c, denstheta_c, nx, ny, nz, hs, acc, result);
+  else cfl_kernel<double><<<grid, kCellThreads, 0, st>>>((const double *)state, dens_c, denstheta_c, nx, ny, nz, hs, acc, result);
   return cudaGetLastError();
 }
 

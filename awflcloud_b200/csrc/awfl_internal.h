@@ -98,9 +98,6 @@ struct SweepArgs32;
 cudaError_t launch_sweep_fp32(int ord, int dir, const SweepArgs32 &A, cudaStream_t st);
 cudaError_t launch_apply_fp32(float *state, float *comp, const float *tend, float dt, int nx, int ny, int nz, int hs,
                               int nsm, cudaStream_t st);
-cudaError_t launch_cfl_fp32(const float *state, const double *dens_c, const double *denstheta_c, double cfl, double dx,
-                            double dy, double dz, int nx, int ny, int nz, int hs, int nsm, unsigned long long *d_out,
-                            cudaStream_t st);
 cudaError_t upload_tables_fp32(int ord, const double *recon, const double *c2g, const double *s2g,
                                const double *deriv, const double *idl, double sigma, const double *wts);
 
@@ -161,9 +158,10 @@ cudaError_t launch_apply_fp64(double *state, const double *tend, double dt, int 
                               int nsm, cudaStream_t st);
 // x += dt*0 on the interior of nplanes planes (the sim2d y split's apply of zero tendencies)
 cudaError_t launch_add_zero_fp64(double *p, int nplanes, int nx, int ny, int nz, int hs, int nsm, cudaStream_t st);
-cudaError_t launch_cfl_fp64(const double *state, const double *dens_c, const double *denstheta_c, double cfl,
-                            double dx, double dy, double dz, int nx, int ny, int nz, int hs, int nsm,
-                            unsigned long long *d_out, cudaStream_t st);
+// The largest max|u +- cs|, |v +- cs|, |w +- cs| of a state into result[0..2]; acc: four
+// device words, zero before the first call and after each.
+cudaError_t launch_cfl(const void *state, int fp32, const double *dens_c, const double *denstheta_c, int nx, int ny,
+                       int nz, int hs, int nsm, unsigned long long *acc, double *result, cudaStream_t st);
 cudaError_t launch_init_state_fp64(const InitLaunch &L, cudaStream_t st);
 cudaError_t launch_init_tracers_fp64(const InitLaunch &L, int ntr, cudaStream_t st);
 cudaError_t launch_tracer_fields(const void *state, int fp32, long plane, const double *dens_c,
