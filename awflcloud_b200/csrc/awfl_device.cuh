@@ -435,7 +435,10 @@ __device__ __forceinline__ void cell_recon(const Sten &sten, int kb, const Sweep
     for (int ii = 0; ii < NG; ii++) sr[kt][ii] = srcfill;
 
   // diffTransformEulerCons{X,Y,Z}. Level kt+1 of f and g is still zero where the reference's
-  // Cauchy products read it: those terms are left out.
+  // Cauchy products read it: those terms are left out. The quotients that share no divisor
+  // (here and the flux's sound speed) still go through a reciprocal of their own: the compiler's
+  // division may call a slow path, and keeping 128 registers across that call cost 32-88
+  // bytes of spills (256x256x128 step 4.25 -> 4.08 ms).
 #pragma unroll
   for (int kt = 0; kt < NA - 1; kt++) {
     Sc fl[5][NG];  // the flux of each variable
@@ -478,7 +481,7 @@ __device__ __forceinline__ void cell_recon(const Sten &sten, int kb, const Sweep
 #pragma unroll
       for (int ir = 1; ir <= kt; ir++)
         tg += (kt + 1. - ir) * (GAMMA * g[ir][ii] * q[idT][kt + 1 - ir][ii] - q[idT][ir][ii] * g[kt + 1 - ir][ii]);
-      g[kt + 1][ii] = (g0 + divk(tg, kt + 1)) / q[idT][0][ii];
+      g[kt + 1][ii] = divp(g0 + divk(tg, kt + 1), make_rcp<Sc>(q[idT][0][ii]));
     }
   }
   rec.series(q);
@@ -537,7 +540,7 @@ __device__ __forceinline__ void riemann(const Sc (&qL)[5], const Sc (&qR)[5], in
     t = 0.5 * (divp(qL[4], rl) + divp(qR[4], rg));
   }
   const Sc p = C0 * pow_gamma(r * t);
-  const Sc cs2 = GAMMA * p / r;
+  const Sc cs2 = divp(GAMMA * p, make_rcp<Sc>(r));
   const Sc cs = sqrt(cs2);
   const Sc vn = vel[DIR], va = vel[TA], vb = vel[TB];
   const Rcp<Sc> rt = make_rcp<Sc>(t), rt2 = rcp_twice(rt), rc2 = make_rcp<Sc>(2. * cs);
