@@ -21,6 +21,9 @@
 #include <cmath>
 
 #include "awfl_internal.h"
+#if defined(__CUDACC__)
+#include "awfl_pow.cuh"
+#endif
 #include "awfl_tv.h"
 
 #if defined(__CUDACC__)
@@ -47,6 +50,15 @@ AWFL_AHD double arcp(double x) {
   return fma(y, fma(-x, y, 1.0), y);
 #else
   return 1. / x;
+#endif
+}
+
+// x^GAMMA: on the device the path's own (a third of the CUDA math library's pow)
+AWFL_AHD double apow_gamma(double x) {
+#if defined(__CUDA_ARCH__)
+  return pow_gamma_cr(x);
+#else
+  return ::pow(x, GAMMA);
 #endif
 }
 
@@ -249,11 +261,93 @@ AWFL_AHD void gll_fwd(const Tables<ORD> &T, const double (&s)[ORD], bool doweno,
   }
 }
 
+// The reverse of the ord-5 WENO reconstruction to GLL values in stencil differences (w5,
+// awfl_internal.h): lu += (d out / d u)^T lout. The same function as gll_vjp's general route
+// through weno_vjp, whose matrices it does not multiply: about 200 FP64 instructions instead
+// of 900, and the FP64 pipe bounds the kernel (64x64x32: 45 -> 28 us per
+// split).
+AWFL_AHD void gll5_vjp(const double (&u)[5], const double (&lout)[3], double (&lu)[5]) {
+  using namespace w5;
+  constexpr double eps = 1.0e-20;
+  // ---- forward
+  const double d0 = u[1] - u[0], d1 = u[2] - u[1], d2 = u[3] - u[2], d3 = u[4] - u[3];
+  const double s[3] = {d1 - d0, d2 - d1, d3 - d2};
+  const double a[3] = {d1 + .5 * s[0], d1 + .5 * s[1], d2 - .5 * s[2]};
+  const double S = s[0] + s[2], g = s[2] - s[0];
+  const double e0 = kE0S * S + kE01 * s[1], h1 = a[1] + kH1 * g, h2 = kH2S * S + kH21 * s[1], h3 = kH3 * g,
+               h4 = kH4 * S - 2 * kH4 * s[1];
+  double t[4];
+  AWFL_UNROLL for (int i = 0; i < 3; i++) t[i] = a[i] * a[i] + (13. / 12) * (s[i] * s[i]);
+  const double avg = (t[0] + t[1] + t[2]) * (1. / 3);
+  const double raw = h1 * (h1 + .5 * h3) + 39.1125 * (h3 * h3) + h2 * ((13. / 3) * h2 + 4.2 * h4) + 625.8 * (h4 * h4);
+  t[3] = avg + (raw - avg) * kSigma;
+  double w0[4], dd[4], S1 = eps;
+  AWFL_UNROLL for (int i = 0; i < 4; i++) {
+    dd[i] = arcp(t[i] * t[i] + eps);
+    w0[i] = (i == 1 ? kD1 : (i == 3 ? kD3 : kD0)) * dd[i];
+    S1 += w0[i];
+  }
+  const double r1 = arcp(S1);
+  double x[4], w[4], dm[4], S2 = eps;
+  AWFL_UNROLL for (int i = 0; i < 4; i++) {
+    const double d = i == 1 ? kD1 : (i == 3 ? kD3 : kD0);
+    x[i] = w0[i] * r1;
+    const double N = (d + d * d) + x[i] * (x[i] - 3. * d), rD = arcp(d * d + x[i] * (1. - 2. * d));
+    w[i] = x[i] * N * rD;
+    dm[i] = ((N + x[i] * (2. * x[i] - 3. * d)) - w[i] * (1. - 2. * d)) * rD;  // d w / d x
+    S2 += w[i];
+  }
+  const double r2 = arcp(S2);
+  AWFL_UNROLL for (int i = 0; i < 4; i++) w[i] *= r2;
+  // ---- reverse: out = (ev - od, mid, ev + od), od = P/2, mid = u[2] + w3 e0 - Q/24,
+  // ev = mid + Q/8 + w3 (h2/4 + h4/16), Q = sum w_i s_i, P = sum w_i a_i + w3 (h1 + h3/4)
+  const double lev = lout[0] + lout[2], lmid = lout[1] + lev, lP = .5 * (lout[2] - lout[0]);
+  const double lQ = .125 * lev - (1. / 24) * lmid;
+  double lw[4], ls[3], la[3];
+  AWFL_UNROLL for (int i = 0; i < 3; i++) {
+    lw[i] = lQ * s[i] + lP * a[i];
+    ls[i] = w[i] * lQ;
+    la[i] = w[i] * lP;
+  }
+  lw[3] = lmid * e0 + lev * (.25 * h2 + .0625 * h4) + lP * (h1 + .25 * h3);
+  const double le0 = w[3] * lmid;
+  double lh1 = w[3] * lP, lh3 = .25 * lh1, lh2 = .25 * (w[3] * lev), lh4 = .25 * lh2;
+  double dot = 0.;
+  AWFL_UNROLL for (int i = 0; i < 4; i++) dot += lw[i] * w[i];
+  AWFL_UNROLL for (int i = 0; i < 4; i++) lw[i] = r2 * (lw[i] - dot) * dm[i];
+  dot = 0.;
+  AWFL_UNROLL for (int i = 0; i < 4; i++) dot += lw[i] * x[i];
+  AWFL_UNROLL for (int i = 0; i < 4; i++) lw[i] = -2. * t[i] * w0[i] * dd[i] * (r1 * (lw[i] - dot));  // of t_i
+  const double lt3 = kSigma * lw[3], llo = ((1. - kSigma) / 3) * lw[3];
+  AWFL_UNROLL for (int i = 0; i < 3; i++) {
+    const double lt = lw[i] + llo;
+    la[i] += 2. * lt * a[i];
+    ls[i] += (13. / 6) * lt * s[i];
+  }
+  lh1 += lt3 * (2. * h1 + .5 * h3);
+  lh3 += lt3 * (.5 * h1 + 78.225 * h3);
+  lh2 += lt3 * ((26. / 3) * h2 + 4.2 * h4);
+  lh4 += lt3 * (4.2 * h2 + 1251.6 * h4);
+  const double lS = kE0S * le0 + kH2S * lh2 + kH4 * lh4, lg = kH1 * lh1 + kH3 * lh3;
+  la[1] += lh1;
+  ls[0] += lS - lg + .5 * la[0];
+  ls[1] += kE01 * le0 + kH21 * lh2 - 2 * kH4 * lh4 + .5 * la[1];
+  ls[2] += lS + lg - .5 * la[2];
+  const double ld1 = la[0] + la[1] + ls[0] - ls[1], ld2 = la[2] + ls[1] - ls[2];
+  lu[0] += ls[0];
+  lu[1] -= ls[0] + ld1;
+  lu[2] += lmid + ld1 - ld2;
+  lu[3] += ld2 - ls[2];
+  lu[4] += ls[2];
+}
+
 template <int ORD>
 AWFL_AHD void gll_vjp(const Tables<ORD> &T, const double (&s)[ORD], bool doweno,
                       const double (&lout)[OrdTraits<ORD>::NGLL], double (&ls)[ORD]) {
   constexpr int NG = OrdTraits<ORD>::NGLL;
-  if (doweno) {
+  if (ORD == 5 && doweno) {
+    if constexpr (ORD == 5) gll5_vjp(s, lout, ls);
+  } else if (doweno) {
     double lc[ORD];
     AWFL_UNROLL for (int m = 0; m < ORD; m++) {
       double t = 0.;
@@ -328,7 +422,7 @@ AWFL_AHD void cell_dt(const Tables<ORD> &T, int kb, const CellArgs &A, CellFwd<O
     const double rr = arcp(X.q[idR][0][ii]);
     const double mn = X.q[NM][0][ii] * rr;
     AWFL_UNROLL for (int x = 0; x < 4; x++) X.f[x][0][ii] = mn * X.q[x + 1][0][ii];
-    X.g[0][ii] = ::pow(X.q[idT][0][ii], GAMMA);
+    X.g[0][ii] = apow_gamma(X.q[idT][0][ii]);
   }
   if (DIR == 2) {
     const double fill = -(X.q[idR][0][NG - 1] - A.dens_g[kb * NG + NG - 1]) * GRAV;
@@ -571,7 +665,7 @@ AWFL_AHD void riemann_fwd(const double (&qL)[5], const double (&qR)[5], double (
     AWFL_UNROLL for (int k = 0; k < 3; k++) vel[k] = 0.5 * (qL[k + 1] * rl + qR[k + 1] * rr);
     t = 0.5 * (qL[4] * rl + qR[4] * rr);
   }
-  const double p = C0 * ::pow(r * t, GAMMA);
+  const double p = C0 * apow_gamma(r * t);
   const double cs = ::sqrt(GAMMA * p * arcp(r));
   const double vn = vel[DIR], va = vel[TA], vb = vel[TB];
   const double rt = arcp(t), rc = 0.5 * arcp(cs);
@@ -584,7 +678,7 @@ AWFL_AHD void riemann_fwd(const double (&qL)[5], const double (&qR)[5], double (
   const double QAv = w2 + va * (w5 + w6), QBv = w3 + vb * (w5 + w6), Q4 = t * (w5 + w6);
   const double r0 = arcp(Q0);
   F[0] = QNv;
-  F[QN] = QNv * QNv * r0 + C0 * ::pow(Q4, GAMMA);
+  F[QN] = QNv * QNv * r0 + C0 * apow_gamma(Q4);
   F[QA] = QNv * QAv * r0;
   F[QB] = QNv * QBv * r0;
   F[4] = QNv * Q4 * r0;
@@ -607,7 +701,7 @@ AWFL_AHD void riemann_vjp(const double (&qL)[5], const double (&qR)[5], const do
     AWFL_UNROLL for (int k = 0; k < 3; k++) vel[k] = 0.5 * (qL[k + 1] * rl + qR[k + 1] * rrr);
     t = 0.5 * (qL[4] * rl + qR[4] * rrr);
   }
-  const double p = C0 * ::pow(r * t, GAMMA);
+  const double p = C0 * apow_gamma(r * t);
   const double cs = ::sqrt(GAMMA * p * arcp(r));
   const double vn = vel[DIR], va = vel[TA], vb = vel[TB];
   const double rt = arcp(t), rc = 0.5 * arcp(cs);
@@ -621,7 +715,7 @@ AWFL_AHD void riemann_vjp(const double (&qL)[5], const double (&qR)[5], const do
   const double QNv = vn * w1 + (vn - cs) * w5 + (vn + cs) * w6;
   const double QAv = w2 + va * W, QBv = w3 + vb * W, Q4 = t * W;
   const double r0 = arcp(Q0);
-  const double pw = ::pow(Q4, GAMMA);
+  const double pw = apow_gamma(Q4);
   // ---- reverse: fluxes -> characteristic state
   const double lQN = lF[0] + lF[QN] * 2. * QNv * r0 + (lF[QA] * QAv + lF[QB] * QBv + lF[4] * Q4) * r0;
   const double lQ0 = -(lF[QN] * QNv * QNv + lF[QA] * QNv * QAv + lF[QB] * QNv * QBv + lF[4] * QNv * Q4) * r0 * r0;

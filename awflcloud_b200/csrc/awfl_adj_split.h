@@ -67,12 +67,22 @@ template <int DIR> AWFL_AHD long fidx(const SplitArgs &A, int i, int j, int k, i
   if (DIR == 1) return ((long)k * (A.ny + 1) + f) * A.nx + i;
   return ((long)f * A.ny + j) * A.nx + i;
 }
-AWFL_AHD void decode_cell(const SplitArgs &A, long c, int &i, int &j, int &k) {
-  i = (int)(c % A.nx);
-  const long r = c / A.nx;
-  j = (int)(r % A.ny);
-  k = (int)(r / A.ny);
+// (x, y, z) of a flat index over extents ex (fastest) and ey, in 32-bit arithmetic where it
+// fits (a 64-bit division is a call of about a hundred instructions)
+AWFL_AHD void unflat(long c, int ex, int ey, int &x, int &y, int &z) {
+  if (c < (1L << 31)) {
+    const unsigned u = (unsigned)c, r = u / (unsigned)ex, q = r / (unsigned)ey;
+    x = (int)(u - r * (unsigned)ex);
+    y = (int)(r - q * (unsigned)ey);
+    z = (int)q;
+  } else {
+    const long r = c / ex;
+    x = (int)(c - r * ex);
+    y = (int)(r % ey);
+    z = (int)(r / ey);
+  }
 }
+AWFL_AHD void decode_cell(const SplitArgs &A, long c, int &i, int &j, int &k) { unflat(c, A.nx, A.ny, i, j, k); }
 
 // ---- edges of one cell (forward recomputation of the linearisation point)
 template <int ORD, int DIR> AWFL_AHD void split_edges(const Tables<ORD> &T, const SplitArgs &A, long c) {
@@ -117,22 +127,9 @@ template <int ORD, int DIR> AWFL_AHD void split_edges(const Tables<ORD> &T, cons
 template <int DIR> AWFL_AHD void split_face(const SplitArgs &A, long idx) {
   const int L = line_len<DIR>(A);
   int i = 0, j = 0, k = 0, f;
-  if (DIR == 0) {
-    f = (int)(idx % (A.nx + 1));
-    const long r = idx / (A.nx + 1);
-    j = (int)(r % A.ny);
-    k = (int)(r / A.ny);
-  } else if (DIR == 1) {
-    i = (int)(idx % A.nx);
-    const long r = idx / A.nx;
-    f = (int)(r % (A.ny + 1));
-    k = (int)(r / (A.ny + 1));
-  } else {
-    i = (int)(idx % A.nx);
-    const long r = idx / A.nx;
-    j = (int)(r % A.ny);
-    f = (int)(r / A.ny);
-  }
+  if (DIR == 0) unflat(idx, A.nx + 1, A.ny, f, j, k);
+  else if (DIR == 1) unflat(idx, A.nx, A.ny + 1, i, f, k);
+  else unflat(idx, A.nx, A.ny, i, j, f);
   const bool periodic = A.ca.bc == BC_PERIODIC;
   const long n = ncell_of(A);
   int ii, jj, kk;
@@ -211,7 +208,7 @@ template <int ORD, int DIR> AWFL_AHD void split_weno(const Tables<ORD> &T, const
   constexpr int NG = OrdTraits<ORD>::NGLL;
   constexpr int NM = 1 + DIR;
   const long n = ncell_of(A);
-  const int v = (int)(idx / n);
+  const int v = (int)(idx >= n) + (idx >= 2 * n) + (idx >= 3 * n) + (idx >= 4 * n);
   const long c = idx - v * n;
   int i, j, k;
   decode_cell(A, c, i, j, k);

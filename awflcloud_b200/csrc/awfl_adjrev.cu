@@ -76,10 +76,9 @@ __global__ void zero_halo_kernel(double *lam, int nx, int ny, int nz, int hs) {
 }
 
 static unsigned grid_for(long n, int nsm) {
-  long b = (n + kAdjThreads - 1) / kAdjThreads;
-  const long cap = (long)nsm * 16;
-  if (b > cap) b = cap;
-  return (unsigned)(b < 1 ? 1 : b);
+  (void)nsm;
+  const long b = (n + kAdjThreads - 1) / kAdjThreads, most = 0x7fffffffL;  // one index per thread
+  return (unsigned)(b < 1 ? 1 : (b < most ? b : most));
 }
 
 template <int ORD, int DIR>

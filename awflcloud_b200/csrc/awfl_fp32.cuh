@@ -208,22 +208,6 @@ __device__ __forceinline__ void weno_coefs32(const T (&u)[ORD], T (&aw)[ORD]) {
     }
   }
 }
-// Ideal weights and relaxation of ord 5 (WenoLimiter.h:28-90) as compile-time constants (the
-// uploaded tables are compared with them), and what the routine below derives from them.
-namespace w5 {
-constexpr double kSum = 2 * 1. + 73.564225445964 + 1584.89319246111;
-// the weights of the side parabolas, of the centred one and of the bridge polynomial
-constexpr double kD0 = 1. / kSum, kD1 = 73.564225445964 / kSum, kD3 = 1584.89319246111 / kSum;
-constexpr double kSigma = 0.73564225445964;
-// the bridge polynomial (quartic minus the idl-weighted parabolas, over idl[3]) in the
-// differences below: e0 = E0S*S + E01*s1, h1 = c + H1*g, h2 = H2S*S + H21*s1, h3 = H3*g,
-// h4 = H4*(S - 2 s1)
-constexpr double kE0S = (3. / 640 + kD0 / 24) / kD3, kE01 = (-1. / 24 - 6. / 640 + kD1 / 24) / kD3;
-constexpr double kH1 = (-5. / 48 + kD0 / 2) / kD3;
-constexpr double kH2S = (-1. / 16 - kD0 / 2) / kD3, kH21 = (.625 - kD1 / 2) / kD3;
-constexpr double kH3 = 1 / (12 * kD3), kH4 = 1 / (24 * kD3);
-}  // namespace w5
-
 // The ord-5 WENO reconstruction to the three GLL points in differences of the stencil: with
 // d_i = u[i+1]-u[i] and s_i = d[i+1]-d[i], the three parabolas are u[2] - s_i/24 + a_i x +
 // (s_i/2) x^2 and the bridge polynomial has the few coefficients of w5, where the matrix

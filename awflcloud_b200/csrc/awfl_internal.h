@@ -26,6 +26,25 @@ template <int ORD> struct OrdTraits;
 template <> struct OrdTraits<5> { static constexpr int NGLL = 3; };
 template <> struct OrdTraits<9> { static constexpr int NGLL = 5; };
 
+// Ideal weights and relaxation of ord 5 (WenoLimiter.h:28-90) as compile-time constants (the
+// uploaded tables are compared with them), and what the reconstruction in stencil
+// differences (FP32: weno_gll5, adjoint: gll5_vjp) derives from them: with d_i = u[i+1] -
+// u[i], s_i = d[i+1] - d[i], S = s_0 + s_2, g = s_2 - s_0, the parabolas are u[2] - s_i/24 +
+// a_i x + (s_i/2) x^2 with a = (d_1 + s_0/2, d_1 + s_1/2, d_2 - s_2/2).
+namespace w5 {
+constexpr double kSum = 2 * 1. + 73.564225445964 + 1584.89319246111;
+// the weights of the side parabolas, of the centred one and of the bridge polynomial
+constexpr double kD0 = 1. / kSum, kD1 = 73.564225445964 / kSum, kD3 = 1584.89319246111 / kSum;
+constexpr double kSigma = 0.73564225445964;
+// the bridge polynomial (quartic minus the idl-weighted parabolas, over idl[3]) in the
+// differences: u[2] + e0, then h1..h4, with e0 = E0S*S + E01*s1, h1 = a_1 + H1*g,
+// h2 = H2S*S + H21*s1, h3 = H3*g, h4 = H4*(S - 2 s1)
+constexpr double kE0S = (3. / 640 + kD0 / 24) / kD3, kE01 = (-1. / 24 - 6. / 640 + kD1 / 24) / kD3;
+constexpr double kH1 = (-5. / 48 + kD0 / 2) / kD3;
+constexpr double kH2S = (-1. / 16 - kD0 / 2) / kD3, kH21 = (.625 - kD1 / 2) / kD3;
+constexpr double kH3 = 1 / (12 * kD3), kH4 = 1 / (24 * kD3);
+}  // namespace w5
+
 // Constant tables (Spatial:274-315), one set per order, uploaded once per device.
 template <int ORD> struct Tables {
   static constexpr int HS = (ORD - 1) / 2;

@@ -59,6 +59,9 @@ template <int ORD> bool complete_tables(Tables<ORD> &t) {
   }
   for (int ii = 0; ii < NG; ii++) ok = ok && t.c2g[ii] == 1.0;
   if (ORD == 5) {
+    const double d[4] = {w5::kD0, w5::kD1, w5::kD0, w5::kD3};
+    for (int i = 0; i < 4; i++) ok = ok && std::fabs(t.idl[i] - d[i]) <= 1e-15;
+    ok = ok && t.sigma == w5::kSigma;
     static const double low[3][3][3] = {{{-kW24, .5, .5}, {2 * kW24, -2., -1.}, {kW2324, 1.5, .5}},
                                         {{-kW24, -.5, .5}, {kW1312, 0., -1.}, {-kW24, .5, .5}},
                                         {{kW2324, -1.5, .5}, {2 * kW24, 2., -1.}, {-kW24, -.5, .5}}};

@@ -6,6 +6,7 @@
 #include <cstdlib>
 #include <random>
 
+#include "awfl_adj.h"
 #include "awfl_device.cuh"
 #include "awfl_recip.h"
 
@@ -114,6 +115,35 @@ template <int ORD> static long check_weno(long n) {
   return bad;
 }
 
+// the ord-5 reconstruction's reverse in stencil differences against the general one (weno_vjp
+// of the GLL projection's transpose): the same derivative, so equal up to rounding, which the
+// weights amplify at most by the ratio of the smoothness indicators' scales: 1e-9 of the
+// largest adjoint for stencils of one scale with jumps
+static long check_gll5_vjp(long n) {
+  std::mt19937_64 g(8);
+  std::uniform_real_distribution<double> u(-1.0, 1.0);
+  long bad = 0;
+  for (long i = 0; i < n; i++) {
+    double s[5], lo[3], la[5] = {0, 0, 0, 0, 0}, lb[5] = {0, 0, 0, 0, 0}, lc[5];
+    const double scale = pow(10.0, 3 * u(g)), slope = u(g), wave = i % 3 == 0 ? 1.0 : (i % 3 == 1 ? 0.1 : 0.0);
+    for (int k = 0; k < 5; k++) s[k] = scale * (slope * k + wave * u(g) + (i % 2 && k > 2 ? 1.0 : 0.0));
+    for (int k = 0; k < 3; k++) lo[k] = u(g);
+    for (int m = 0; m < 5; m++) {
+      lc[m] = 0;
+      for (int k = 0; k < 3; k++) lc[m] += c_tab5.c2g[m * 3 + k] * lo[k];
+    }
+    adj::gll5_vjp(s, lo, la);
+    adj::weno_vjp<5>(c_tab5, s, lc, lb);
+    double top = 0, off = 0;
+    for (int k = 0; k < 5; k++) {
+      top = fmax(top, fabs(lb[k]));
+      off = fmax(off, fabs(la[k] - lb[k]));
+    }
+    if (!(off <= 1e-9 * top) && bad++ < 5) printf("FAIL gll5_vjp %g of %g\n", off, top);
+  }
+  return bad;
+}
+
 template <int ORD> static bool load_tables(const char *path, Tables<ORD> &T) {
   FILE *f = fopen(path, "rb");
   if (!f) return false;
@@ -131,7 +161,7 @@ int main(int argc, char **argv) {
   }
   const long scale = argc > 3 ? atol(argv[3]) : 1;
   const long bad = check_pow(2000000 * scale) + check_div(1000000 * scale) + check_weno<5>(1000000 * scale) +
-                   check_weno<9>(200000 * scale);
+                   check_weno<9>(200000 * scale) + check_gll5_vjp(200000 * scale);
   if (!bad) printf("ok\n");
   return bad ? 1 : 0;
 }

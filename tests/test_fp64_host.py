@@ -1,7 +1,8 @@
 """CPU checks of the FP64 path's short forms (awfl_pow.cuh, awfl_div.cuh, awfl_device.cuh),
 compiled for the host with g++: each equals the general routine it stands in for bit for
 bit -- the pressure's pow, the quotients, the WENO reconstruction -- at the edges of its
-range and for the values that fall back to the general routine."""
+range and for the values that fall back to the general routine; and the reconstruction's
+reverse in stencil differences (awfl_adj.h) equals the general one up to rounding."""
 import os
 import shutil
 import subprocess
