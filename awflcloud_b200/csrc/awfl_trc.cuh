@@ -237,12 +237,13 @@ __global__ void __launch_bounds__(128, AWFL_TRC_LIMIT_MINB) tracer_limit_faces_k
 // in order, a face keeps the first pass's value unless a face it reads (min of face f-1 for
 // un > 0; min of face 0 and max of face 1 for face n with un < 0) now holds a value other
 // than the unscaled one the first pass read; only those faces are limited again. The warp
-// loads 32 faces at a time (one per lane) and runs the walk over them uniformly, the
-// values coming by shuffle: the loads of a chunk overlap instead of one chain of
-// dependent loads per face.
+// loads 32 faces at a time (one per lane) and knows by ballot which of them read a face that
+// changed, so it steps from one such face to the next instead of through all of them
+// (128x128x64, three tracers: 14 -> 7 us per split).
 template <class TA, int DIR>
 __global__ void __launch_bounds__(128) tracer_limit_lines_kernel(TA T, int hs) {
   using Fx = typename TA::Flux;
+  constexpr unsigned kAll = 0xffffffffu;
   const Geo<DIR> G(T.A, hs);
   const int n = G.n();
   const int lane = threadIdx.x & 31;
@@ -264,50 +265,59 @@ __global__ void __launch_bounds__(128) tracer_limit_lines_kernel(TA T, int hs) {
     };
     const Fx *TF = T.TF + l * nf;
     Fx *TF2 = T.TF2 + l * nf;
-    Fx sprev = 0, uprev = 0;              // the face behind: serial (scaled) and unscaled values
-    Fx s0 = 0, u0 = 0, s1 = 0, u1 = 0;   // faces 0 and 1, likewise
+    auto redo = [&](Fx F, Fx f1, Fx f2, int c) {  // face flux F limited by its upwind cell c
+      int ck, cj, ci;
+      G.at(k0, j0, i0, c, ck, cj, ci);
+      return limit_face(T, F, f1, f2, T.tr[l * G.sv + G.g(ck, cj, ci)], T.D[G.cell(ck, cj, ci)] + trc_dens(T, hs, ck));
+    };
+    Fx sprev = 0, uprev = 0;            // the face behind the chunk: serial (scaled) and unscaled
+    Fx s0 = 0, u0 = 0, s1 = 0, u1 = 0;  // faces 0 and 1, likewise
     for (int base = 0; base <= n; base += 32) {
       const int fme = base + lane;
+      const bool in = fme <= n;
       long fim = 0;
       Fx Fm = 0, Tm = 0, Um = 0;
-      if (fme <= n) {
+      if (in) {
         fim = face(fme);
         Fm = TF[fim];
         Tm = TF2[fim];
         Um = T.UN[fim];
       }
-      const int cnt = n + 1 - base < 32 ? n + 1 - base : 32;
-      for (int i = 0; i < cnt; i++) {
-        const int f = base + i;
-        const Fx F = __shfl_sync(0xffffffffu, Fm, i);
-        Fx out = __shfl_sync(0xffffffffu, Tm, i);
-        const Fx un = __shfl_sync(0xffffffffu, Um, i);
-        int c = -1;
-        Fx f1 = 0, f2 = 0;
-        if (un > 0 && f > 0) {
-          if (!(dmin(sprev, Fx(0)) == dmin(uprev, Fx(0)))) {  // upwind cell f-1 reads face f-1
-            c = f - 1;
-            f1 = dmin(sprev, Fx(0));
-            f2 = dmax(F, Fx(0));
-          }
-        } else if (un < 0 && f == n) {
-          if (!(dmin(s0, Fx(0)) == dmin(u0, Fx(0))) || (n >= 2 && !(dmax(s1, Fx(0)) == dmax(u1, Fx(0))))) {
-            c = 0;  // upwind cell 0
-            f1 = dmin(s0, Fx(0));
-            f2 = dmax(n == 1 ? F : s1, Fx(0));
-          }
+      // readers: faces upwinded from the cell behind; changed: faces whose min moved
+      const unsigned readers = __ballot_sync(kAll, in && Um > 0 && fme > 0);
+      unsigned changed = __ballot_sync(kAll, !(dmin(Tm, Fx(0)) == dmin(Fm, Fx(0))));
+      const unsigned carry = !(dmin(sprev, Fx(0)) == dmin(uprev, Fx(0)));
+      unsigned from = 0;  // lanes below it are done
+      for (;;) {
+        const unsigned need = readers & ((changed << 1) | carry) & (from < 32 ? kAll << from : 0u);
+        if (!need) break;
+        const int i = __ffs(need) - 1;
+        const Fx sb = __shfl_sync(kAll, Tm, i > 0 ? i - 1 : 0);
+        const Fx F = __shfl_sync(kAll, Fm, i);
+        const Fx out = redo(F, dmin(i > 0 ? sb : sprev, Fx(0)), dmax(F, Fx(0)), base + i - 1);
+        if (lane == i) {
+          Tm = out;
+          TF2[fim] = out;
         }
-        if (c >= 0) {
-          int ck, cj, ci;
-          G.at(k0, j0, i0, c, ck, cj, ci);
-          out = limit_face(T, F, f1, f2, T.tr[l * G.sv + G.g(ck, cj, ci)], T.D[G.cell(ck, cj, ci)] + trc_dens(T, hs, ck));
+        changed = (changed & ~(1u << i)) | ((unsigned)!(dmin(out, Fx(0)) == dmin(F, Fx(0))) << i);
+        from = (unsigned)i + 1;
+      }
+      if (base == 0) {
+        s0 = __shfl_sync(kAll, Tm, 0);
+        u0 = __shfl_sync(kAll, Fm, 0);
+        s1 = __shfl_sync(kAll, Tm, 1);
+        u1 = __shfl_sync(kAll, Fm, 1);
+      }
+      if (n - base < 32) {  // face n: upwinded from cell 0, it reads faces 0 and 1
+        const int i = n - base;
+        const Fx un = __shfl_sync(kAll, Um, i), F = __shfl_sync(kAll, Fm, i);
+        if (un < 0 && (!(dmin(s0, Fx(0)) == dmin(u0, Fx(0))) || (n >= 2 && !(dmax(s1, Fx(0)) == dmax(u1, Fx(0)))))) {
+          const Fx out = redo(F, dmin(s0, Fx(0)), dmax(n == 1 ? F : s1, Fx(0)), 0);
           if (lane == i) TF2[fim] = out;
         }
-        sprev = out;
-        uprev = F;
-        if (f == 0) { s0 = out; u0 = F; }
-        if (f == 1) { s1 = out; u1 = F; }
       }
+      sprev = __shfl_sync(kAll, Tm, 31);
+      uprev = __shfl_sync(kAll, Fm, 31);
     }
   }
 }
