@@ -138,7 +138,7 @@ __device__ __forceinline__ double limit_face(const TracerArgs &T, double F, doub
 __device__ __forceinline__ double trc_update(const TracerArgs &T, double q, int hs, int k, long c, double Fl,
                                              double Fr) {
   const double dens = T.D[c] + T.A.dens_c[hs + k];
-  const double tend = -(Fr - Fl) / T.A.dxd;
+  const double tend = div_known_any(Fr - Fl, -T.A.dxd, T.A.nrdx_h, T.A.nrdx_l);  // -(Fr - Fl) / dx
   return q * dens + T.A.dt * tend;  // Spatial:952-953, then Temporal_ader.h:67-69
 }
 
@@ -168,24 +168,24 @@ namespace {
 #ifndef AWFL_TRC_CELL_MINB
 #define AWFL_TRC_CELL_MINB 8
 #endif
-// One thread per cell and tracer; the blocks of one run of 128 cells are consecutive for
-// the tracers (block b: cells (b / ntr) * 128 .., tracer b % ntr), so the recorded series
-// that they share is read from DRAM once.
+// One thread per cell and tracer, cells plane by plane (blockIdx.y: the plane); the blocks of
+// one run of 128 cells are consecutive for the tracers, so the recorded series that they
+// share is read from DRAM once.
 template <int ORD, int DIR>
 __global__ void __launch_bounds__(128, ORD == 5 ? AWFL_TRC_CELL_MINB : 1) tracer_cell_kernel(TracerArgs T) {
   constexpr int HS = (ORD - 1) / 2;
   constexpr int NG = OrdTraits<ORD>::NGLL;
   const SweepArgs &A = T.A;
   const Geo<DIR> G(A, HS);
-  const unsigned ncell = (unsigned)G.nz * G.ny * G.nx;
+  const unsigned plane = (unsigned)G.nx * G.ny, ncell = plane * G.nz;
   const unsigned cb = blockIdx.x / (unsigned)T.ntr;
-  const int l = (int)(blockIdx.x - cb * (unsigned)T.ntr);
-  const unsigned c = cb * blockDim.x + threadIdx.x;
-  if (c >= ncell) return;
+  const int l = (int)(blockIdx.x - cb * (unsigned)T.ntr), k = (int)blockIdx.y;
+  const unsigned pq = cb * 128u + threadIdx.x;
+  if (pq >= plane) return;
+  const unsigned c = k * plane + pq;
   if (l == 0 && c < G.nlines()) T.flag[c] = 0;  // the limiter's per-line flags (ncell >= nlines)
   if (l == 0 && c == 0) *T.count = 0;
-  int i, j, k;
-  unflat(c, G.nx, G.ny, k, j, i);
+  const int j = (int)(pq / (unsigned)G.nx), i = (int)(pq - (unsigned)j * G.nx);
   const int p0 = DIR == 0 ? i : (DIR == 1 ? j : k);
   const int n = G.n();
   const bool posdef = (T.pos >> l) & 1ull;
@@ -287,13 +287,12 @@ cudaError_t run(const TracerArgs &T, int io, cudaStream_t st) {
   constexpr int HS = (ORD - 1) / 2;
   constexpr int NG = OrdTraits<ORD>::NGLL;
   const SweepArgs &A = T.A;
-  const long ncell = (long)A.nz * A.ny * A.nx;
-  const long nf = (long)(A.nz + (DIR == 2)) * (A.ny + (DIR == 1)) * (A.nx + (DIR == 0));
-  const unsigned gc = (unsigned)((ncell + 127) / 128), gf = (unsigned)((nf + 127) / 128);
+  const long plane = (long)A.ny * A.nx;
+  const dim3 gc = plane_grid(plane, A.nz), gf = plane_grid((long)(A.ny + (DIR == 1)) * (A.nx + (DIR == 0)), A.nz + (DIR == 2));
   if (!(io & TRC_IN_DIVIDED)) tracer_divide_kernel<TracerArgs><<<gc, 128, 0, st>>>(T, HS);
   cudaError_t e = launch_sweep_t<P64Trc, ORD, DIR>(A, st);  // state split + records
   if (e != cudaSuccess) return e;
-  tracer_cell_kernel<ORD, DIR><<<gc * (unsigned)T.ntr, 128, 0, st>>>(T);
+  tracer_cell_kernel<ORD, DIR><<<dim3(gc.x * (unsigned)T.ntr, (unsigned)A.nz), 128, 0, st>>>(T);
   const long nlines = DIR == 0 ? (long)A.nz * A.ny : (DIR == 1 ? (long)A.nz * A.nx : (long)A.ny * A.nx);
   tracer_limit_faces_kernel<TracerArgs, DIR><<<gf, 128, 0, st>>>(T, HS);
   const long lw = (nlines * T.ntr + 3) / 4;  // one warp per flagged line and tracer, grid-strided

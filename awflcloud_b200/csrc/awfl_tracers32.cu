@@ -316,12 +316,11 @@ cudaError_t run32(const TracerArgs32 &T, int io, cudaStream_t st) {
   constexpr int NG = OrdTraits<ORD>::NGLL;
   const SweepArgs32 &A = T.A;
   const long ncell = (long)A.nz * A.ny * A.nx;
-  const long nf = (long)(A.nz + (DIR == 2)) * (A.ny + (DIR == 1)) * (A.nx + (DIR == 0));
-  const unsigned gc = (unsigned)((ncell + 127) / 128), gf = (unsigned)((nf + 127) / 128);
+  const dim3 gc = plane_grid((long)A.ny * A.nx, A.nz), gf = plane_grid((long)(A.ny + (DIR == 1)) * (A.nx + (DIR == 0)), A.nz + (DIR == 2));
   if (!(io & TRC_IN_DIVIDED)) tracer_divide_kernel<TracerArgs32><<<gc, 128, 0, st>>>(T, HS);
   cudaError_t e = launch_sweep_t<P32Trc, ORD, DIR>(A, st);  // state split + records
   if (e != cudaSuccess) return e;
-  tracer_cell32_kernel<ORD, DIR><<<gc, 128, 0, st>>>(T);
+  tracer_cell32_kernel<ORD, DIR><<<(unsigned)((ncell + 127) / 128), 128, 0, st>>>(T);
   const long nlines = DIR == 0 ? (long)A.nz * A.ny : (DIR == 1 ? (long)A.nz * A.nx : (long)A.ny * A.nx);
   tracer_limit_faces_kernel<TracerArgs32, DIR><<<gf, 128, 0, st>>>(T, HS);
   const long lw = (nlines * T.ntr + 3) / 4;  // one warp per flagged line and tracer, grid-strided
