@@ -110,14 +110,13 @@ void tiles(const awfl_config &c, int dir, int W, int *nbx, int *nby) {
 
 // The shape an untuned ensemble starts with: the cheapest of the candidates by the sweeps' cost
 // model (awfl_sweep.cuh) over the members' tiles, spread over the SMs and at least as long
-// as the longest line, times what the shape costs on a full chip (measured, 24 members of
-// 32..96 cells a side: FP32 us per launch x 327 343 237 262, y 239 242 228 237, z 262 294
-// 243 284 in the candidates' order; FP64 x 865 1054 741 766, y 774 757 844 822, z 875 890 931
-// 1000). That ensemble: FP32 1.63 -> 1.40 ms for two steps, FP64 4.99 -> 4.72; 4 members of
-// 16..40: FP32 0.114 -> 0.099.
+// as the longest line, times what the shape costs on a full chip (measured, 24 and 64 members
+// of 32..128 cells a side; us per launch of 24, in the candidates' order: FP32 x 278 286 212
+// 228, y 233 223 222 222, z 237 258 236 256; FP64 x 760 952 687 689, y 713 674 786 770, z 743
+// 770 878 931). Against the first candidates, 24 members, FP32: 1.63 -> 1.40 ms for two steps.
 int default_shape(const awfl_ensemble *e, int dir) {
-  static const double f32[3][4] = {{1.38, 1.45, 1.0, 1.1}, {1.05, 1.06, 1.0, 1.04}, {1.08, 1.2, 1.0, 1.17}};
-  static const double f64[3][4] = {{1.17, 1.42, 1.0, 1.03}, {1.02, 1.0, 1.11, 1.09}, {1.0, 1.02, 1.07, 1.15}};
+  static const double f32[3][4] = {{1.32, 1.38, 1.0, 1.08}, {1.02, 1.03, 1.0, 1.02}, {1.01, 1.11, 1.0, 1.1}};
+  static const double f64[3][4] = {{1.11, 1.39, 1.0, 1.02}, {1.02, 1.0, 1.17, 1.15}, {1.0, 1.04, 1.18, 1.25}};
   if (e->ord != 5) return 0;
   int best = 0;
   double cost = 0;
@@ -135,8 +134,9 @@ int default_shape(const awfl_ensemble *e, int dir) {
       longest = std::max(longest, chunks);
     }
     const double k = std::min(4.0, std::ceil(ctas / e->nsm));  // resident per SM
-    const double c = (e->prec == AWFL_FP32 ? f32 : f64)[dir][s] * (0.6 + 0.4 * k) *
-                     std::max(longest, k > 0 ? units / (k * e->nsm) : 0.0);
+    double len = 0;  // chunks a CTA runs: its share, and half a tile more where the tiles come in rounds
+    if (ctas > 0) len = units / (k * e->nsm) + (ctas > k * e->nsm ? 0.5 * units / ctas : 0.0);
+    const double c = (e->prec == AWFL_FP32 ? f32 : f64)[dir][s] * (0.6 + 0.4 * k) * std::max(longest, len);
     if (s == 0 || c < cost) { best = s; cost = c; }
   }
   return best;
@@ -148,10 +148,11 @@ int build_lists(awfl_ensemble *e, const std::vector<void *> &states, void **d_ou
                 EnsList<SweepArgs32> (&l32)[3]) {
   const int n = (int)e->mem.size();
   const size_t asz = e->prec == AWFL_FP32 ? sizeof(SweepArgs32) : sizeof(SweepArgs);
-  // layout per direction: args[n] | prefix[n+1] | nbx[n], 64-byte aligned pieces (the
+  // layout per direction: args[n] | prefix[n+1] | nbx[n] | two words, 64-byte aligned pieces (the
   // FP32 arguments hold a 64-byte-aligned tensor map field)
   auto up64 = [](size_t x) { return (x + 63) & ~size_t(63); };
-  const size_t per = up64(asz * n) + up64(sizeof(long) * (n + 1)) + up64(sizeof(int) * n);
+  const size_t at_nbx = up64(asz * n) + up64(sizeof(long) * (n + 1)), at_sched = at_nbx + up64(sizeof(int) * n);
+  const size_t per = at_sched + 64;
   std::vector<unsigned char> host(per * 3, 0);
   for (int dir = 0; dir < 3; dir++) {
     int C, W;
@@ -165,7 +166,7 @@ int build_lists(awfl_ensemble *e, const std::vector<void *> &states, void **d_ou
     unsigned char *base = host.data() + per * dir;
     unsigned char *pa = base;
     long *pp = (long *)(base + up64(asz * n));
-    int *pn = (int *)(base + up64(asz * n) + up64(sizeof(long) * (n + 1)));
+    int *pn = (int *)(base + at_nbx);
     long total = 0;
     for (size_t q = 0; q < order.size(); q++) {
       const int m = order[q];
@@ -201,7 +202,8 @@ int build_lists(awfl_ensemble *e, const std::vector<void *> &states, void **d_ou
     l64[dir].args = (const SweepArgs *)base;
     l32[dir].args = (const SweepArgs32 *)base;
     l64[dir].prefix = l32[dir].prefix = (const long *)(base + up64(asz * n));
-    l64[dir].nbx = l32[dir].nbx = (const int *)(base + up64(asz * n) + up64(sizeof(long) * (n + 1)));
+    l64[dir].nbx = l32[dir].nbx = (const int *)(base + at_nbx);
+    l64[dir].sched = l32[dir].sched = (unsigned *)(base + at_sched);
   }
   *d_out = d;
   return AWFL_OK;
