@@ -183,18 +183,6 @@ __device__ __forceinline__ void sweep_tile(const typename P::Args &A, const int 
   // of pitch RW with line w at column HS + w. Other chunks (and a tile whose wait gave
   // up) use cp.async. Out-of-range box elements (the last tile's missing lines) read as
   // zero and are never used.
-  static_assert(!TMA || ASYNC, "the TMA path feeds the async ring");
-  constexpr int RW = (TMA && DIR != 0) ? tma_ring_pitch<ORD, C, W, (int)sizeof(Real)>() : W;
-  static_assert(!TMA || DIR != 0 || ((C * W * (int)sizeof(Real)) % 128 == 0 && (2 * HS * (int)sizeof(Real)) % 16 == 0 &&
-                                     (C * (int)sizeof(Real)) % 16 == 0),
-                "x-sweep TMA pages must be 128-byte multiples starting at 16-byte-aligned x");
-  static_assert(!TMA || DIR == 0 || (W * (int)sizeof(Real)) % 16 == 0, "y/z-sweep TMA boxes start at x = bx*W");
-  constexpr int NM = 1 + DIR;
-  static_assert((C & (C - 1)) == 0 && C >= 2 * HS, "chunk must be a power of two >= 2*HS");
-  // Register path: load the next chunk's rows before the reconstruction (latency hidden
-  // behind it, at the cost of 5 live registers) for the z sweep, whose loads stride over
-  // whole planes; after the updates for x and y, where occupancy matters more (measured).
-  constexpr bool EARLY_PREFETCH = !ASYNC && DIR == 2;
   // The C cells of a chunk of one line are C consecutive lanes of one warp (x sweep: a
   // warp holds 32/C lines along x; y/z sweeps: 32/C neighbouring lines, so that a warp's
   // global accesses are 32/C consecutive x cells in each of C rows), so the interface
@@ -206,7 +194,25 @@ __device__ __forceinline__ void sweep_tile(const typename P::Args &A, const int 
   // memory would otherwise touch C rows instead of 32/W (FP64 z split measured 3.61 ->
   // 3.71 ms with the shuffles).
   constexpr bool SHFL = C <= 32 && (C * W) % 32 == 0 && (DIR == 0 || ASYNC);
-
+  static_assert(!TMA || ASYNC, "the TMA path feeds the async ring");
+  // Row pitch of a y/z ring. A warp of the shuffle path reads LW = 32/C neighbouring words of
+  // each of C rows; with the pitch an odd multiple of LW the rows start in different banks
+  // (at pitch W, a multiple of the banks, all C of them in the same ones: FP64 256x256x128,
+  // y 1343 -> 1299 us, z 1420 -> 1376; ord 9, 128x128x64, y 875 -> 837, z 909 -> 862).
+  constexpr int LW = C <= 32 ? 32 / C : 1;
+  constexpr int RW = DIR == 0 ? W
+                     : TMA    ? tma_ring_pitch<ORD, C, W, (int)sizeof(Real)>()
+                     : (SHFL && W % LW == 0) ? (W / LW % 2 ? W : W + LW) : W;
+  static_assert(!TMA || DIR != 0 || ((C * W * (int)sizeof(Real)) % 128 == 0 && (2 * HS * (int)sizeof(Real)) % 16 == 0 &&
+                                     (C * (int)sizeof(Real)) % 16 == 0),
+                "x-sweep TMA pages must be 128-byte multiples starting at 16-byte-aligned x");
+  static_assert(!TMA || DIR == 0 || (W * (int)sizeof(Real)) % 16 == 0, "y/z-sweep TMA boxes start at x = bx*W");
+  constexpr int NM = 1 + DIR;
+  static_assert((C & (C - 1)) == 0 && C >= 2 * HS, "chunk must be a power of two >= 2*HS");
+  // Register path: load the next chunk's rows before the reconstruction (latency hidden
+  // behind it, at the cost of 5 live registers) for the z sweep, whose loads stride over
+  // whole planes; after the updates for x and y, where occupancy matters more (measured).
+  constexpr bool EARLY_PREFETCH = !ASYNC && DIR == 2;
   __shared__ __align__(128) Real ring[5][R * RW];
   __shared__ __align__(8) unsigned long long mbar;  // TMA path only
   __shared__ int sAbort;                            // TMA path: a wait of this tile gave up
