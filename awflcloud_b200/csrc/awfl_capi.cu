@@ -484,8 +484,9 @@ int awfl_create(const awfl_config *cfg, int device, awfl_ctx **out) {
 
   int rc = set_device(c);
   if (rc) { g_create_error = c->err; delete c; return rc; }
-  cudaDeviceProp prop;
-  if (cudaGetDeviceProperties(&prop, device) == cudaSuccess) c->nsm = prop.multiProcessorCount;
+  // one attribute, not cudaGetDeviceProperties: that was most of a context's creation time
+  int nsm = 0;
+  if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && nsm > 0) c->nsm = nsm;
   rc = ensure_tables(c);
   if (rc) { g_create_error = c->err; delete c; return rc; }
   const int nz = cfg->nz, g = c->ngll;
