@@ -34,7 +34,6 @@
 #include "awfl_fp32_args.h"
 #include "awfl_pow.cuh"
 #include "awfl_sweep.cuh"
-#include "awfl_tv.h"
 
 namespace awfl {
 
@@ -67,17 +66,9 @@ __device__ __forceinline__ float binom_gamma_m1(float x) {
 }
 
 template <int ORD> struct Tables32 {
-  static constexpr int HS = (ORD - 1) / 2;
   static constexpr int NG = OrdTraits<ORD>::NGLL;
-  float recon[ORD * ORD * ORD];
-  // the high-order candidate's coefficients straight from the stencil: (its full-stencil
-  // map minus the idl-weighted low-order candidates' maps) / idl[hs+1], formed in FP64
-  float hi[ORD * ORD];
-  float c2g[ORD * NG];
   float s2g[ORD * NG];
   float deriv[NG * NG];
-  float idl[HS + 2];
-  float sigma;
   float wts[NG];
 };
 // One copy per translation unit that includes this header (awfl_fp32.cu, awfl_ens32.cu),
@@ -87,11 +78,6 @@ static __constant__ Tables32<9> c32_tab9;
 template <int ORD> __device__ __forceinline__ const Tables32<ORD> &tab32();
 template <> __device__ __forceinline__ const Tables32<5> &tab32<5>() { return c32_tab5; }
 template <> __device__ __forceinline__ const Tables32<9> &tab32<9>() { return c32_tab9; }
-
-template <int N> __device__ __forceinline__ float tv_evalf(const float *a);
-template <> __device__ __forceinline__ float tv_evalf<3>(const float *a) { return awfl_tv_n3<float>(a); }
-template <> __device__ __forceinline__ float tv_evalf<5>(const float *a) { return awfl_tv_n5<float>(a); }
-template <> __device__ __forceinline__ float tv_evalf<9>(const float *a) { return awfl_tv_n9<float>(a); }
 
 // Two independent FP32 lanes evaluated with the paired sm_100 instructions (FFMA2, FMUL2,
 // FADD2: one instruction, two results, each rounded like the scalar operation), so that
@@ -129,158 +115,19 @@ __device__ __forceinline__ F2 fmaT(F2 a, float b, F2 c) { return F2(__ffma2_rn(a
 __device__ __forceinline__ float rcpT(float x) { return frcp(x); }
 __device__ __forceinline__ F2 rcpT(F2 x) { return F2(frcp(x.v.x), frcp(x.v.y)); }
 
-template <int N> __device__ __forceinline__ F2 tv_evalf2(const F2 *a) {
-  if constexpr (N == 3) return awfl_tv_n3<F2>(a);
-  else if constexpr (N == 5) return awfl_tv_n5<F2>(a);
-  else return awfl_tv_n9<F2>(a);
-}
-template <int N> __device__ __forceinline__ float tv_evalT(const float *a) { return tv_evalf<N>(a); }
-template <int N> __device__ __forceinline__ F2 tv_evalT(const F2 *a) { return tv_evalf2<N>(a); }
+}  // namespace awfl
 
-// WenoLimiter.h:93-172 in FP32.
-template <int ORD, class T>
-__device__ __forceinline__ void weno_coefs32(const T (&u)[ORD], T (&aw)[ORD]) {
-  constexpr int HS = (ORD - 1) / 2;
-  const Tables32<ORD> &Tb = tab32<ORD>();
-  const float eps = 1.0e-20f;
-  // Structural zeros (symmetric stencils; checked when the tables are uploaded) are left
-  // out: the centred low-order candidate's odd coefficients and the high-order map's odd
-  // coefficients take nothing from the stencil's centre value.
-  T a[HS + 2][ORD];
-#pragma unroll
-  for (int i = 0; i < HS + 1; i++)
-#pragma unroll
-    for (int ii = 0; ii < HS + 1; ii++) {
-      T acc = T(0.f);
-#pragma unroll
-      for (int s = 0; s < HS + 1; s++) {
-        if (HS % 2 == 0 && i == HS / 2 && s == HS / 2 && ii % 2 == 1) continue;
-        acc = fmaT(Tb.recon[(i * ORD + s) * ORD + ii], u[i + s], acc);
-      }
-      a[i][ii] = acc;
-    }
-#pragma unroll
-  for (int ii = 0; ii < ORD; ii++) {
-    T acc = T(0.f);
-#pragma unroll
-    for (int s = 0; s < ORD; s++) {
-      if (s == HS && ii % 2 == 1) continue;
-      acc = fmaT(Tb.hi[s * ORD + ii], u[s], acc);
-    }
-    a[HS + 1][ii] = acc;
-  }
-  T tv[HS + 2];
-#pragma unroll
-  for (int i = 0; i < HS + 1; i++) tv[i] = tv_evalT<HS + 1>(a[i]);
-  tv[HS + 1] = tv_evalT<ORD>(a[HS + 1]);
-  T lo_avg = T(0.f);
-#pragma unroll
-  for (int i = 0; i < HS + 1; i++) lo_avg += tv[i];
-  lo_avg = lo_avg * (1.0f / (HS + 1));
-  tv[HS + 1] = fmaT(tv[HS + 1] - lo_avg, Tb.sigma, lo_avg);
-  T wts[HS + 2];
-  T sum = T(0.f);
-#pragma unroll
-  for (int i = 0; i < HS + 2; i++) {
-    wts[i] = Tb.idl[i] * rcpT(fmaT(tv[i], tv[i], T(eps)));
-    sum += wts[i];
-  }
-  T inv = rcpT(sum + eps);
-  sum = T(0.f);
-#pragma unroll
-  for (int i = 0; i < HS + 2; i++) {
-    const T w = wts[i] * inv;
-    const float d = Tb.idl[i];
-    const T num = w * fmaT(w, w + (-3.f * d), T(d + d * d));
-    wts[i] = num * rcpT(fmaT(w, 1.f - 2.f * d, T(d * d)));
-    sum += wts[i];
-  }
-  inv = rcpT(sum + eps);
-#pragma unroll
-  for (int ii = 0; ii < ORD; ii++) aw[ii] = T(0.f);
-#pragma unroll
-  for (int i = 0; i < HS + 2; i++) {
-    const T w = wts[i] * inv;
-#pragma unroll
-    for (int ii = 0; ii < ORD; ii++) {
-      if (i < HS + 1 && ii > HS) continue;  // zero coefficients of the low-order candidates
-      aw[ii] = fmaT(w, a[i][ii], aw[ii]);
-    }
-  }
-}
-// The ord-5 WENO reconstruction to the three GLL points in differences of the stencil: with
-// d_i = u[i+1]-u[i] and s_i = d[i+1]-d[i], the three parabolas are u[2] - s_i/24 + a_i x +
-// (s_i/2) x^2 and the bridge polynomial has the few coefficients of w5, where the matrix
-// form (weno_coefs32) multiplies 49 entries. Equal in exact arithmetic, the weights summing
-// to one; about 100 FP32 instructions instead of 150, and u[2] enters the values unrounded.
-// The sweep is issue-bound: with the time series on point pairs
-// (Pts below), 1,500 -> 1,130 instructions per cell and split, 256x256x128 step 1.433 -> 1.200 ms.
-template <class T> __device__ __forceinline__ void weno_gll5(const T (&u)[5], T (&out)[3]) {
-  using namespace w5;
-  const T d0 = u[1] - u[0], d1 = u[2] - u[1], d2 = u[3] - u[2], d3 = u[4] - u[3];
-  const T s0 = d1 - d0, s1 = d2 - d1, s2 = d3 - d2;
-  const T a0 = fmaT(.5f, s0, d1), c = fmaT(.5f, s1, d1), a2 = fmaT(-.5f, s2, d2);
-  const T S = s0 + s2, g = s2 - s0;
-  const T e0 = fmaT((float)kE0S, S, (float)kE01 * s1);
-  const T h1 = fmaT((float)kH1, g, c);
-  const T h2 = fmaT((float)kH2S, S, (float)kH21 * s1);
-  const T h3 = (float)kH3 * g;
-  const T h4 = fmaT((float)kH4, S, (float)(-2 * kH4) * s1);
-  // smoothness indicators (coefs_to_tv of the parabolas and of the bridge polynomial)
-  const float k13 = (float)(13. / 12);
-  const T t0 = fmaT(a0, a0, (k13 * s0) * s0), t1 = fmaT(c, c, (k13 * s1) * s1), t2 = fmaT(a2, a2, (k13 * s2) * s2);
-  T t3 = fmaT(h1, fmaT(.5f, h3, h1), (39.1125f * h3) * h3);
-  t3 = fmaT(h2, fmaT(4.2f, h4, (float)(13. / 3) * h2), t3);
-  t3 = fmaT(625.8f * h4, h4, t3);
-  const T avg = (t0 + t1 + t2) * (float)(1. / 3);
-  t3 = fmaT(t3 - avg, (float)kSigma, avg);
-  // weights idl/(tv^2 + eps), up to the common factor idl[0] that the normalisation drops
-  const T eps = T(1.0e-20f);
-  T w[4] = {rcpT(fmaT(t0, t0, eps)), (float)(kD1 / kD0) * rcpT(fmaT(t1, t1, eps)), rcpT(fmaT(t2, t2, eps)),
-            (float)(kD3 / kD0) * rcpT(fmaT(t3, t3, eps))};
-  T inv = rcpT(((w[0] + w[1]) + (w[2] + w[3])) + eps);
-#pragma unroll
-  for (int i = 0; i < 4; i++) {  // map_weights (WenoLimiter.h:12-17)
-    const double d = i == 1 ? kD1 : (i == 3 ? kD3 : kD0);
-    const T x = w[i] * inv;
-    w[i] = (x * fmaT(x, x + (float)(-3 * d), T((float)(d + d * d)))) * rcpT(fmaT(x, (float)(1 - 2 * d), T((float)(d * d))));
-  }
-  inv = rcpT(((w[0] + w[1]) + (w[2] + w[3])) + eps);
-  const T Q = fmaT(w[0], s0, fmaT(w[1], s1, w[2] * s2));
-  const T P = fmaT(w[0], a0, fmaT(w[1], c, fmaT(w[2], a2, w[3] * fmaT(.25f, h3, h1))));
-  const T mid = fmaT(inv, fmaT((float)(-1. / 24), Q, w[3] * e0), u[2]);
-  const T ev = fmaT(inv, fmaT(.125f, Q, w[3] * fmaT(.0625f, h4, .25f * h2)), mid);
-  const T od = (.5f * inv) * P;
-  out[0] = ev - od;
-  out[1] = mid;
-  out[2] = ev + od;
-}
+#include "awfl_weno32.h"
+
+namespace awfl {
 
 template <int ORD, class T>
 __device__ __forceinline__ void reconstruct_gll32(const T (&sten)[ORD], T (&out)[OrdTraits<ORD>::NGLL], bool doweno) {
   constexpr int NG = OrdTraits<ORD>::NGLL;
   const Tables32<ORD> &Tb = tab32<ORD>();
-  if (ORD == 5 && doweno) {
+  if (doweno) {
     if constexpr (ORD == 5) weno_gll5(sten, out);
-  } else if (doweno) {
-    T wc[ORD];
-    weno_coefs32<ORD>(sten, wc);
-    // polynomial coefficients -> values at the GLL points, which sit symmetrically about
-    // the cell centre (x = 0): the centre takes the constant coefficient alone, the mirror
-    // points x and -x the even part plus and minus the odd part
-    static_assert(NG % 2 == 1, "an odd number of GLL points, one at the centre");
-    out[NG / 2] = wc[0];
-#pragma unroll
-    for (int ii = 0; ii < NG / 2; ii++) {
-      const int jr = NG - 1 - ii;
-      T ev = T(0.f), od = T(0.f);
-#pragma unroll
-      for (int s = 0; s < ORD; s += 2) ev = fmaT(Tb.c2g[s * NG + jr], wc[s], ev);
-#pragma unroll
-      for (int s = 1; s < ORD; s += 2) od = fmaT(Tb.c2g[s * NG + jr], wc[s], od);
-      out[jr] = ev + od;
-      out[ii] = ev - od;
-    }
+    else weno_gll9(sten, out);
   } else {
 #pragma unroll
     for (int ii = 0; ii < NG; ii++) {
@@ -359,6 +206,9 @@ template <int NG> __device__ __forceinline__ Pts<NG> same(float x) {
 // centre; at ord 5 it is {-3 4 -1; -1 0 1; 1 -4 3})
 template <int ORD> __device__ __forceinline__ Pts<OrdTraits<ORD>::NGLL> deriv32(const Pts<OrdTraits<ORD>::NGLL> &x, float sc) {
   constexpr int NG = OrdTraits<ORD>::NGLL;
+  constexpr double kD[3][5] = {{-10, 13.51300497744848, -16. / 3, 2.8203283558848535, -1},
+                               {-2.4819805060619657, 0, 3.4914862437758787, -1.5275252316519454, 0.5180194939380343},
+                               {.75, -2.6731691553909065, 0, 2.6731691553909065, -.75}};
   Pts<NG> r;
   if constexpr (ORD == 5) {
     const float x0 = x.get(0), x1 = x.c, x2 = x.get(2);
@@ -366,17 +216,15 @@ template <int ORD> __device__ __forceinline__ Pts<OrdTraits<ORD>::NGLL> deriv32(
     r.set(1, x2 - x0);
     r.set(2, fmaf(-4.f, x1, fmaf(3.f, x2, x0)));
   } else {
-    const Tables32<ORD> &T = tab32<ORD>();
-#pragma unroll
-    for (int ii = 0; ii < NG; ii++) {
-      float acc = 0.f;
-#pragma unroll
-      for (int s = 0; s < NG; s++) {
-        if (ii == NG / 2 && s == NG / 2) continue;
-        acc = fmaf(T.deriv[s * NG + ii], x.get(s), acc);
-      }
-      r.set(ii, acc);
-    }
+    // the rows of mirror points are each other's reverse negated: lane y takes the same
+    // coefficients on the reversed values, and -sc (128x128x64 step 0.483 -> 0.476 ms)
+    auto rev = [](F2 a) { return F2(a.v.y, a.v.x); };
+    const F2 p0 = x.p[0], p1 = x.p[1], m0 = rev(p0), m1 = rev(p1), cc = F2(x.c), pm = F2(sc, -sc);
+    r.p[0] = pm * fmaT((float)kD[0][0], p0, fmaT((float)kD[0][1], p1, fmaT((float)kD[0][2], cc, fmaT((float)kD[0][3], m1, (float)kD[0][4] * m0))));
+    r.p[1] = pm * fmaT((float)kD[1][0], p0, fmaT((float)kD[1][2], cc, fmaT((float)kD[1][3], m1, (float)kD[1][4] * m0)));
+    const F2 h = fmaT((float)kD[2][0], p0, (float)kD[2][1] * p1);
+    r.c = sc * (h.v.x - h.v.y);
+    return r;
   }
   return sc * r;
 }
@@ -686,53 +534,32 @@ static inline cudaError_t upload_tables32_here(int ord, const double *recon, con
                                                const double *deriv, const double *idl, double sigma,
                                                const double *wts) {
   auto fill = [&](auto &t, int o, int g) {
-    const int hs = (o - 1) / 2;
-    for (int i = 0; i < o * o * o; i++) t.recon[i] = (float)recon[i];
-    for (int sidx = 0; sidx < o; sidx++)
-      for (int ii = 0; ii < o; ii++) {
-        double m = recon[((hs + 1) * o + sidx) * o + ii];
-        if (ii <= hs)
-          for (int i = 0; i <= hs; i++)
-            if (sidx - i >= 0 && sidx - i <= hs) m -= idl[i] * recon[(i * o + (sidx - i)) * o + ii];
-        t.hi[sidx * o + ii] = (float)(m / idl[hs + 1]);
-      }
-    for (int i = 0; i < o * g; i++) { t.c2g[i] = (float)c2g[i]; t.s2g[i] = (float)s2g[i]; }
+    for (int i = 0; i < o * g; i++) t.s2g[i] = (float)s2g[i];
     for (int i = 0; i < g * g; i++) t.deriv[i] = (float)deriv[i];
-    for (int i = 0; i < hs + 2; i++) t.idl[i] = (float)idl[i];
-    t.sigma = (float)sigma;
     for (int i = 0; i < g; i++) t.wts[i] = (float)wts[i];
   };
-  // the structural zeros and symmetries the FP32 reconstruction leaves out of its sums
-  auto structure_ok = [&](const auto &t, int o, int g) {
-    const int hs = (o - 1) / 2;
-    double dmax = 0, rmax = 0;
-    for (int x = 0; x < g * g; x++) dmax = fmax(dmax, fabs((double)t.deriv[x]));
-    for (int x = 0; x < o * o * o; x++) rmax = fmax(rmax, fabs((double)t.recon[x]));
-    bool ok = g % 2 == 1 && hs % 2 == 0 && t.c2g[0 * g + g / 2] == 1.f &&
-              fabs((double)t.deriv[(g / 2) * g + g / 2]) <= 1e-6 * dmax;
-    for (int sidx = 1; sidx < o; sidx++) ok = ok && t.c2g[sidx * g + g / 2] == 0.f;
-    for (int sidx = 0; sidx < o; sidx++)
-      for (int ii = 0; ii < g; ii++)
-        ok = ok && t.c2g[sidx * g + ii] == ((sidx % 2) ? -1.f : 1.f) * t.c2g[sidx * g + (g - 1 - ii)];
-    double hmax = 0;
-    for (int x = 0; x < o * o; x++) hmax = fmax(hmax, fabs((double)t.hi[x]));
-    for (int ii = 1; ii < o; ii += 2) {
-      ok = ok && fabs((double)t.hi[hs * o + ii]) <= 1e-6 * hmax;
-      if (ii <= hs) ok = ok && fabs((double)t.recon[((hs / 2) * o + hs / 2) * o + ii]) <= 1e-6 * rmax;
-    }
-    return ok;
-  };
+  // what the FP32 forms take as compile-time constants, against the tables they come from
+  auto near = [](double a, double b) { return fabs(a - b) <= 1e-12 * fmax(1.0, fabs(b)); };
+  bool ok = near(deriv[(ord == 5 ? 1 : 2) * (ord == 5 ? 3 : 5) + (ord == 5 ? 1 : 2)], 0.0);
   if (ord == 5) {
     Tables32<5> t;
     fill(t, 5, 3);
-    if (!structure_ok(t, 5, 3)) return cudaErrorInvalidValue;
-    for (int i = 0; i < 4; i++)  // the reconstruction's compile-time weights
-      if (fabs(idl[i] - (i == 1 ? w5::kD1 : (i == 3 ? w5::kD3 : w5::kD0))) > 1e-12 || fabs(sigma - w5::kSigma) > 1e-12) return cudaErrorInvalidValue;
+    ok = ok && near(sigma, w5::kSigma);
+    for (int i = 0; i < 4; i++) ok = ok && near(idl[i], i == 1 ? w5::kD1 : (i == 3 ? w5::kD3 : w5::kD0));
+    if (!ok) return cudaErrorInvalidValue;
     return cudaMemcpyToSymbol(c32_tab5, &t, sizeof t);
   }
   Tables32<9> t;
   fill(t, 9, 5);
-  if (!structure_ok(t, 9, 5)) return cudaErrorInvalidValue;
+  ok = ok && near(sigma, w9::kSigma) && near(c2g[1 * 5 + 3], w9::kX1) && near(c2g[1 * 5 + 4], 0.5);
+  for (int i = 0; i < 6; i++) ok = ok && near(idl[i], w9::ideal(i));
+  for (int i = 0; i < 9; i++) {
+    // u = 1 in cell 7 (D_2 = 1, D_3 = -5), then in cell 8 (D_3 = 1); P_2 = 0 for both
+    if (i < 5) ok = ok && near(recon[(3 * 9 + 4) * 9 + i], w9::kN.c[i]) && near(recon[(4 * 9 + 4) * 9 + i], w9::kM.c[i]);
+    ok = ok && near(recon[(5 * 9 + 7) * 9 + i], w9::kFa.c[i] - 5 * w9::kFb.c[i]) &&
+         near(recon[(5 * 9 + 8) * 9 + i], w9::kFb.c[i]);
+  }
+  if (!ok) return cudaErrorInvalidValue;
   return cudaMemcpyToSymbol(c32_tab9, &t, sizeof t);
 }
 

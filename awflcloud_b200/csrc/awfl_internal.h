@@ -44,6 +44,37 @@ constexpr double kH1 = (-5. / 48 + kD0 / 2) / kD3;
 constexpr double kH2S = (-1. / 16 - kD0 / 2) / kD3, kH21 = (.625 - kD1 / 2) / kD3;
 constexpr double kH3 = 1 / (12 * kD3), kH4 = 1 / (24 * kD3);
 }  // namespace w5
+// The same for ord 9 (weno_gll9). D_j is the fifth difference over cells j..j+5 of the nine;
+// P_i the quartic through the averages of cells i..i+4.
+namespace w9 {
+constexpr double kSum = 2 * 1. + 2 * 2.15766927997459 + 2.40224886796286 + 1136.12697719888;
+constexpr double kSigma = 0.0288539981181442;
+__host__ __device__ constexpr double ideal(int i) {
+  return (i == 5 ? 1136.12697719888 : (i == 2 ? 2.40224886796286 : (i % 2 ? 2.15766927997459 : 1.))) / kSum;
+}
+constexpr double kX1 = 0.32732683535398857;  // sqrt(3/7)/2: the GLL points are 0, +-kX1, +-1/2
+struct Poly {
+  double c[9];
+  __host__ __device__ constexpr double even(double x) const { return c[0] + x * x * (c[2] + x * x * (c[4] + x * x * (c[6] + x * x * c[8]))); }
+  __host__ __device__ constexpr double odd(double x) const { return x * (c[1] + x * x * (c[3] + x * x * (c[5] + x * x * c[7]))); }
+};
+// P_3 - P_2 = D_2 N(x), P_4 - P_3 = D_3 M(x), P_1 - P_2 = -D_1 N(-x), P_0 - P_1 = -D_0 M(-x)
+constexpr Poly kN = {{3. / 640, 5. / 48, -1. / 16, -1. / 12, 1. / 24, 0, 0, 0, 0}};
+constexpr Poly kM = {{-71. / 1920, -3. / 16, 7. / 16, -1. / 4, 1. / 24, 0, 0, 0, 0}};
+// The octic less P_2: coefficient i is kFa[i] (D_2 -+ D_1) + kFb[i] (D_3 -+ D_0), minus for
+// even i; the bridge polynomial less P_2 (the octic minus the ideal(0..4)-weighted P_i, over
+// ideal(5)) likewise with kHa, kHb.
+constexpr Poly kFa = {{-725. / 688128, 5911. / 215040, 1889. / 129024, -701. / 23040, -127. / 9216, 11. / 1920, 1. / 384,
+                       -1. / 10080, -1. / 13440}};
+constexpr Poly kFb = {{35. / 294912, -3229. / 645120, -3229. / 1935360, 47. / 7680, 47. / 27648, -1. / 640, -7. / 17280,
+                       1. / 10080, 1. / 40320}};
+constexpr Poly bridge(const Poly &f, double d, const Poly &p) {
+  Poly r = {};
+  for (int i = 0; i < 9; i++) r.c[i] = (f.c[i] - d * p.c[i]) / ideal(5);
+  return r;
+}
+constexpr Poly kHa = bridge(kFa, ideal(0) + ideal(1), kN), kHb = bridge(kFb, ideal(0), kM);
+}  // namespace w9
 
 // Constant tables (Spatial:274-315), one set per order, uploaded once per device.
 template <int ORD> struct Tables {

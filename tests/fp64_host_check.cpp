@@ -10,6 +10,12 @@
 #include "awfl_device.cuh"
 #include "awfl_recip.h"
 
+namespace awfl {
+static float fmaT(float a, float b, float c) { return fmaf(a, b, c); }
+static float rcpT(float x) { return 1.f / x; }
+}  // namespace awfl
+#include "awfl_weno32.h"
+
 using namespace awfl;
 
 // pow_gamma_cr(x) == pow_cr(x, GAMMA) bit for bit: the table's range, its ends, bin edges
@@ -144,6 +150,39 @@ static long check_gll5_vjp(long n) {
   return bad;
 }
 
+// the FP32 form's reconstruction in stencil differences against the general routine in FP64:
+// rounding 2^-24 of the stencil's range, times at most 32 in a fifth difference, 4 in 1/tv^2 and
+// 8 in the mapped weights, and the rounding of the values themselves
+template <int ORD> static long check_weno32(long n) {
+  std::mt19937_64 g(9);
+  std::uniform_real_distribution<double> u(-1.0, 1.0);
+  std::normal_distribution<double> nd;
+  long bad = 0;
+  for (long i = 0; i < n; i++) {
+    StenV<ORD> s;
+    float f[ORD], o[OrdTraits<ORD>::NGLL];
+    const double scale = pow(10.0, 2 * u(g)), base = i % 2 ? u(g) : 0.0, wave = .1 + .8 * fabs(u(g)), phase = 3 * u(g);
+    const int jump = (int)(g() % ORD);
+    double range = 0, top = 0;
+    for (int k = 0; k < ORD; k++) {
+      const double x = i % 3 == 0 ? nd(g) : (i % 3 == 1 ? sin(wave * k + phase) : (k >= jump) + .01 * nd(g));
+      f[k] = (float)(scale * (base + (i % 5 ? x : 0.01 * x)));
+      s.v[k] = f[k];
+    }
+    for (int k = 0; k < ORD; k++) {
+      range = fmax(range, fabs(s.v[k] - s.v[ORD / 2]));
+      top = fmax(top, fabs(s.v[k]));
+    }
+    const GllV<ORD> r = reconstruct_gll_general<ORD>(s, true);
+    if constexpr (ORD == 5) weno_gll5<float>(f, o);
+    else weno_gll9<float>(f, o);
+    for (int k = 0; k < OrdTraits<ORD>::NGLL; k++)
+      if (!(fabs(o[k] - r.v[k]) <= 0x1p-24 * (1024 * range + 2 * top)) && bad++ < 5)
+        printf("FAIL weno32 ord %d point %d: %g %g range %g\n", ORD, k, o[k], r.v[k], range);
+  }
+  return bad;
+}
+
 template <int ORD> static bool load_tables(const char *path, Tables<ORD> &T) {
   FILE *f = fopen(path, "rb");
   if (!f) return false;
@@ -161,7 +200,8 @@ int main(int argc, char **argv) {
   }
   const long scale = argc > 3 ? atol(argv[3]) : 1;
   const long bad = check_pow(2000000 * scale) + check_div(1000000 * scale) + check_weno<5>(1000000 * scale) +
-                   check_weno<9>(200000 * scale) + check_gll5_vjp(200000 * scale);
+                   check_weno<9>(200000 * scale) + check_gll5_vjp(200000 * scale) +
+                   check_weno32<5>(400000 * scale) + check_weno32<9>(400000 * scale);
   if (!bad) printf("ok\n");
   return bad ? 1 : 0;
 }

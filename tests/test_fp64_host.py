@@ -2,7 +2,8 @@
 compiled for the host with g++: each equals the general routine it stands in for bit for
 bit -- the pressure's pow, the quotients, the WENO reconstruction -- at the edges of its
 range and for the values that fall back to the general routine; and the reconstruction's
-reverse in stencil differences (awfl_adj.h) equals the general one up to rounding."""
+reverse in stencil differences (awfl_adj.h) equals the general one up to rounding, as does the
+FP32 form's reconstruction (awfl_weno32.h)."""
 import os
 import shutil
 import subprocess
