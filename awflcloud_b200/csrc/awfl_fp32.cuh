@@ -472,7 +472,9 @@ struct P32 {
   // ord 5: five CTAs of 128 threads per SM (86-93 registers): 256x256x128 step 1.160 ms,
   // against 1.200 at the compiler's 115 (four) and 1.177 at six (80); the small-grid shapes
   // and the x-slab sweep at four (awfl_sweep.cuh)
-  static constexpr int min_blocks(int ord) { return ord == 5 ? 5 : 1; }
+  // ord 9: three (168 registers, no spills by cp.async): 128x128x64 step 0.476 ms at two CTAs,
+  // 0.433 at three
+  static constexpr int min_blocks(int ord) { return ord == 5 ? 5 : 3; }
   using Args = SweepArgs32;
   // rows that TMA cannot address (16-byte pitch) come by cp.async: 107 instead of about 85 us
   // for the x split of 130x100x70
@@ -521,7 +523,19 @@ struct P32 {
 // 401, 8x8 385, 4x16 418; z 4x32 388, 8x16 408, 4x64 511, 4x16 438.
 template <> struct PolicyShape<P32, 5, 0> { static constexpr int C = 8, W = 16; };
 template <> struct PolicyShape<P32, 5, 1> { static constexpr int C = 8, W = 16; };
+// Ord 9, three CTAs of 128 threads (128x128x64, us): x 32 x 4 138, 8 x 16 154; y 16 x 8 141,
+// 8 x 16 157; z 8 x 16 141, 16 x 8 149. With the shapes for small grids, against 32 x 2, 8 x 16
+// and 8 x 16 for all: step 32x32x16 45 -> 33 us, 64x64x32 92 -> 77, 97x61x45 197 (two CTAs) -> 150,
+// 400x1x200 184 (two) -> 48, 128x128x64 433 -> 418.
+template <> struct PolicyShape<P32, 9, 0> { static constexpr int C = 32, W = 4; };
+template <> struct PolicyShape<P32, 9, 1> { static constexpr int C = 16, W = 8; };
 // The shapes for small grids (PolicyShapes, awfl_sweep.cuh).
+template <int DIR> struct PolicyShapes<P32, 9, DIR> {
+  static constexpr int n = DIR == 0 ? 2 : 3;
+  static constexpr int C[3] = {DIR == 1 ? 8 : 16, DIR == 0 ? 128 : 32, 128}, W[3] = {DIR == 1 ? 16 : 8, DIR == 0 ? 1 : 4, 1};
+  static constexpr double factor[3] = {DIR == 0 ? 1.0 : (DIR == 1 ? 0.92 : 1.12), DIR == 0 ? 1.15 : (DIR == 1 ? 1.12 : 1.25),
+                                       1.4};
+};
 template <int DIR> struct PolicyShapes<P32, 5, DIR> {
   static constexpr int n = 4;
   static constexpr int C[4] = {DIR == 2 ? 8 : 4, 16, 32, 128}, W[4] = {DIR == 2 ? 16 : 32, 8, 4, 1};

@@ -108,12 +108,23 @@ template <int DIR> struct SmallShapes<5, DIR> {
   static constexpr int C[3] = {DIR == 0 ? 8 : 16, 32, 128}, W[3] = {DIR == 0 ? 16 : 8, 4, 1};
   static constexpr double factor[3] = {1.0, 1.0, 1.1};
 };
+// Ord 9: x 32 x 4 (128x128x64, us: 734; 32 x 2 770, 16 x 8 761), and for y and z 8 x 16
+// (840 873), 16 x 8 (795 828) or 32 x 4 (756 826), whichever pads the lines less and fills the
+// chip. Step, all in 32 x 2 (x) or 8 x 16 -> the rule, us: 32x32x16 172 -> 94, 64x64x32 408
+// -> 341, 97x61x45 1004 -> 753, 400x1x200 805 -> 207, 128x128x64 2494 -> 2295, 256x256x64
+// 10130 -> 9415; 80x50x48 571 -> 576.
+template <> struct PolicyShape<P64, 9, 0> { static constexpr int C = 32, W = 4; };
+template <int DIR> struct SmallShapes<9, DIR> {
+  static constexpr int n = DIR == 0 ? 2 : 3;
+  static constexpr int C[3] = {16, DIR == 0 ? 128 : 32, 128}, W[3] = {8, DIR == 0 ? 1 : 4, 1};
+  static constexpr double factor[3] = {DIR == 2 ? 0.99 : 1.0, DIR == 0 ? 1.1 : (DIR == 1 ? 1.0 : 0.93), 1.2};
+};
 template <int ORD, int DIR> struct PolicyShapes<P64, ORD, DIR> : SmallShapes<ORD, DIR> {};
 // The same for the recording policies, whose 20-odd record planes are written along x: a y
 // or z shape of few lines spreads each store over as many rows as it has cells of a line
 // (128x128x64 with tracers, y split, 8 x 16 / 16 x 8 / 32 x 4: 445 / 467 / 497 us; 64x64x32:
 // 121 / 107 / 98).
-template <int ORD, int DIR> struct RecordShapes : SmallShapes<ORD, DIR> {};
+template <int ORD, int DIR> struct RecordShapes { static constexpr int n = 0; };
 template <int DIR> struct RecordShapes<5, DIR> : SmallShapes<5, DIR> {
   static constexpr double factor[3] = {DIR == 0 ? 1.0 : (DIR == 1 ? 1.1 : 1.2), DIR == 0 ? 1.0 : (DIR == 1 ? 1.2 : 1.3),
                                        DIR == 0 ? 1.1 : 1.5};

@@ -724,11 +724,13 @@ cudaError_t launch_sweep_shape(const typename P::Args &A, cudaStream_t st) {
   // the x split of a slab with neighbouring slabs' columns: the SLAB instantiation
   bool slab = false;
   if constexpr (DIR == 0 && P::kSlab && base) slab = A.xh[0] != nullptr || A.xh[1] != nullptr;
-  if constexpr (P::kTmaRing && (DIR == 0 || W >= 16)) {
+  if constexpr (P::kTmaRing && ORD == 5 && (DIR == 0 || W >= 16)) {
     // the policy encodes this launch's tensor map (box = one chunk of one variable); a
     // layout TMA cannot address (alignment) leaves tma off and the cp.async path runs. So do
     // y and z shapes of few lines: the pitch that TMA wants puts their rows in the same banks
-    // (FP32 64x64x32, y split in 16 x 8: 17.4 us, by cp.async 16.6)
+    // (FP32 64x64x32, y split in 16 x 8: 17.4 us, by cp.async 16.6), and ord 9, where TMA's
+    // bookkeeping spills at three CTAs per SM (128x128x64, 32 x 2, 8 x 16 and 8 x 16: 148 168
+    // 155 us, by cp.async 138 158 140)
     typename P::Args a = A;
     if (P::prepare_tma(a, ORD, DIR, C, W)) {
       if constexpr (DIR == 0 && P::kSlab && base)
@@ -745,10 +747,13 @@ cudaError_t launch_sweep_shape(const typename P::Args &A, cudaStream_t st) {
 // the chunk latency of an SM's only CTA: ceil(L/C) chunks, and an epilogue where no lane of
 // the last one is free, each as long as the CTAs that share an SM make it. Measured with the
 // FP64 ord-5 sweep: 5.9 us for one CTA per SM, 8 for two, 10.5 for three, 13 for four, the
-// most; the tiles of a grid take equally long, so an SM runs its share four at a time.
-inline double sweep_cost(int C, int L, long tiles, int nsm, bool ends) {
+// most; the tiles of a grid take equally long, so an SM runs its share `slots` (4) at a time,
+// each CTA after the first adding `share` (0.4) to the latency. Ord 9, two CTAs (FP64) or
+// three (FP32) per SM: 20.5 us for one FP64 CTA, 24.6 for two; FP32 4.4, 5.2 and 6.
+inline double sweep_cost(int C, int L, long tiles, int nsm, bool ends, int slots, double share) {
   const long k = (tiles + nsm - 1) / nsm;  // of the busiest SM
-  return ((L + C - 1) / C + (ends && L % C ? 0.0 : 0.35)) * (k / 4 * 2.2 + (k % 4 ? 0.6 + 0.4 * (k % 4) : 0.0));
+  const double full = 1 + share * (slots - 1), rest = k % slots ? 1 + share * (k % slots - 1) : 0.0;
+  return ((L + C - 1) / C + (ends && L % C ? 0.0 : 0.35)) * (k / slots * full + rest);
 }
 
 // The single-grid sweep of a policy whose PolicyShapes lists further shapes takes its first
@@ -773,9 +778,11 @@ cudaError_t launch_sweep_t(const typename P::Args &A, cudaStream_t st) {
     const int across = DIR == 0 ? A.ny : A.nx;  // lines of one plane, W to a tile
     const long planes = DIR == 2 ? A.ny : A.nz;
     int best = -1;
-    double cost = 0.95 * P::base_factor(A) * sweep_cost(B::C, L, (across + BW - 1) / BW * planes, A.nsm, false);
+    constexpr int slots = ORD == 5 ? 4 : (P::min_blocks(ORD) > 2 ? P::min_blocks(ORD) : 2);
+    constexpr double share = ORD == 5 ? 0.4 : 0.2;
+    double cost = 0.95 * P::base_factor(A) * sweep_cost(B::C, L, (across + BW - 1) / BW * planes, A.nsm, false, slots, share);
     for (int i = 0; i < S::n; i++) {
-      const double c = S::factor[i] * sweep_cost(S::C[i], L, (across + S::W[i] - 1) / S::W[i] * planes, A.nsm, true);
+      const double c = S::factor[i] * sweep_cost(S::C[i], L, (across + S::W[i] - 1) / S::W[i] * planes, A.nsm, true, slots, share);
       if (c < cost) { best = i; cost = c; }
     }
     if constexpr (DIR == 0 && P::kSlab) {

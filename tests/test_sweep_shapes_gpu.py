@@ -96,3 +96,38 @@ def test_fp32_shapes_match_fp64(n, bc):
         a, b = (x[v, h:-h, h:-h, h:-h].double() for x in (d32, d64))
         norm = float(b.norm())
         assert float((a - b).norm()) <= 1e-5 * norm if norm else float(a.norm()) == 0, v
+
+
+# ord 9: 32 x 4, 16 x 8, 8 x 16 and 128 x 1 in every direction, full and ragged
+GRIDS9 = [((32, 32, 16), PPW), ((33, 31, 15), PPP), ((7, 64, 129), WWW), ((130, 5, 9), PPW), ((400, 1, 12), PPP),
+          ((16, 8, 130), PPP), ((64, 64, 32), PPW), ((20, 200, 9), WWW), ((65, 48, 5), PPW)]
+
+
+@pytest.mark.parametrize("n,bc", GRIDS9)
+def test_fp64_ord9_shapes_equal_oracle(n, bc):
+    c, o = _ctx(n, bc, ord_=9), Oracle(*n, bc=bc, ord_=9, crpow=True)
+    st = _state(n, c.hs, 5)
+    d = torch.from_numpy(st).cuda()
+    dt = o.compute_dt(st, 0.5)
+    for _ in range(2):
+        c.step(d, dt)
+        o.time_step(st, dt)
+        assert _bits(d.cpu().numpy(), st)
+
+
+@pytest.mark.parametrize("n,bc", GRIDS9 + [((9, 150, 140), PPP), ((200, 20, 30), WWW)])
+def test_fp32_ord9_shapes_match_fp64(n, bc):
+    c64, c32 = _ctx(n, bc, ord_=9), _ctx(n, bc, ord_=9, precision=capi.FP32)
+    st = _state(n, c64.hs, 6)
+    d32 = c32.new_state()
+    d32[:5] = torch.from_numpy(st).cuda().float()
+    d64 = d32[:5].double()
+    dt = c64.cfl(d64, 0.5)
+    for _ in range(2):
+        c64.step(d64, dt)
+        c32.step(d32, dt)
+    h = c64.hs
+    for v in range(5):
+        a, b = (x[v, h:-h, h:-h, h:-h].double() for x in (d32, d64))
+        norm = float(b.norm())
+        assert float((a - b).norm()) <= 1e-5 * norm if norm else float(a.norm()) == 0, v
