@@ -95,19 +95,16 @@ __device__ __forceinline__ double divp(const double &a, const Rcp<double> &r) {
 // a / r.b, correctly rounded
 template <class Sc> __device__ __forceinline__ Sc divr(const Sc &a, const Rcp<Sc> &r) { return a / r.b; }
 __device__ __forceinline__ double divr(const double &a, const Rcp<double> &r) { return div_markstein(a, r.b, r.y); }
-// a / r.b, correctly rounded for every dividend: nonzero ones below 2^-900 in magnitude
-// (where the quotient or the remainder could leave the normal range, as transported
-// tracer values that decay towards zero can) take the IEEE division itself; a zero
-// dividend stays on the short path, whose RN(a*y) is IEEE's signed zero
+// The divisions of transported tracer values, correctly rounded for every dividend: nonzero
+// ones below 2^-900 in magnitude (where the quotient or the remainder could leave the normal
+// range, as values that decay towards zero can) take the IEEE division itself; a zero
+// dividend stays on the short path, whose quotient is IEEE's signed zero
 // (the test on the bit pattern, off the FP64 pipe)
 __device__ __forceinline__ bool is_tiny(double a) {
   const unsigned h = (unsigned)__double2hiint(a) & 0x7fffffffu;
   return h < ((1023u - 900u) << 20) && (h | (unsigned)__double2loint(a)) != 0;
 }
-__device__ __forceinline__ double divr_any(double a, const Rcp<double> &r) {
-  return is_tiny(a) ? a / r.b : div_markstein(a, r.b, r.y);
-}
-// the same for r.b > 0, and for a divisor b known on the host as 1/b = h + l
+// for r.b > 0, and for a divisor b known on the host as 1/b = h + l
 __device__ __forceinline__ double divp_any(double a, const Rcp<double> &r) { return is_tiny(a) ? a / r.b : divp(a, r); }
 __device__ __forceinline__ double div_known_any(double a, double b, double h, double l) {
   return is_tiny(a) ? a / b : div_known(a, h, l);
@@ -131,7 +128,7 @@ __device__ __forceinline__ double divk(const double &a, int k) {
                 : div_known(a, 0x1.9999999999999p-3, 0x1.3333333333333p-56);  // k == 5
 }
 
-// divk for dividends of any magnitude (divr_any's range)
+// divk for dividends of any magnitude
 __device__ __forceinline__ double divk_any(double a, int k) {
   if (k == 1) return a;
   if ((k & (k - 1)) == 0) return a * (1.0 / k);
