@@ -724,13 +724,15 @@ cudaError_t launch_sweep_shape(const typename P::Args &A, cudaStream_t st) {
   // the x split of a slab with neighbouring slabs' columns: the SLAB instantiation
   bool slab = false;
   if constexpr (DIR == 0 && P::kSlab && base) slab = A.xh[0] != nullptr || A.xh[1] != nullptr;
-  if constexpr (P::kTmaRing && ORD == 5 && (DIR == 0 || W >= 16)) {
+  if constexpr (P::kTmaRing && ORD == 5 && DIR != 2 && base) {
     // the policy encodes this launch's tensor map (box = one chunk of one variable); a
-    // layout TMA cannot address (alignment) leaves tma off and the cp.async path runs. So do
-    // y and z shapes of few lines: the pitch that TMA wants puts their rows in the same banks
-    // (FP32 64x64x32, y split in 16 x 8: 17.4 us, by cp.async 16.6), and ord 9, where TMA's
-    // bookkeeping spills at three CTAs per SM (128x128x64, 32 x 2, 8 x 16 and 8 x 16: 148 168
-    // 155 us, by cp.async 138 158 140)
+    // layout TMA cannot address (alignment) leaves tma off and the cp.async path runs. TMA only
+    // where it is the faster: the x and y shapes of large grids (FP32 256x256x128, us, TMA
+    // 370 384, by cp.async 377 392). The z sweep needs 79 registers by cp.async instead of 89
+    // (383 us, TMA 390); small grids' shapes start sooner (64x64x32 x split 12.4 us, TMA
+    // 14.1) and TMA's pitch puts a narrow shape's rows in the same banks (y 16.6, TMA 17.4);
+    // at ord 9 TMA's bookkeeping spills at three CTAs per SM (128x128x64, 32 x 2, 8 x 16 and
+    // 8 x 16: 148 168 155 us, by cp.async 138 158 140)
     typename P::Args a = A;
     if (P::prepare_tma(a, ORD, DIR, C, W)) {
       if constexpr (DIR == 0 && P::kSlab && base)
