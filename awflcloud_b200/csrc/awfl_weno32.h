@@ -32,11 +32,13 @@ template <class T> __device__ __forceinline__ void weno_gll5(const T (&u)[5], T 
   t3 = fmaT(625.8f * h4, h4, t3);
   const T avg = (t0 + t1 + t2) * (float)(1. / 3);
   t3 = fmaT(t3 - avg, (float)kSigma, avg);
-  // weights idl/(tv^2 + eps), up to the common factor idl[0] that the normalisation drops
+  // weights idl/(tv^2 + eps) over idl[0] (two products fewer), and so is the eps of their
+  // normalisation: w/(sum + eps) is the scheme's whatever the size of the values (from
+  // differences of about 1e3 on, sum is no longer large against eps)
   const T eps = T(1.0e-20f);
   T w[4] = {rcpT(fmaT(t0, t0, eps)), (float)(kD1 / kD0) * rcpT(fmaT(t1, t1, eps)), rcpT(fmaT(t2, t2, eps)),
             (float)(kD3 / kD0) * rcpT(fmaT(t3, t3, eps))};
-  T inv = rcpT(((w[0] + w[1]) + (w[2] + w[3])) + eps);
+  T inv = rcpT(((w[0] + w[1]) + (w[2] + w[3])) + T((float)(1.0e-20 / kD0)));
 #pragma unroll
   for (int i = 0; i < 4; i++) {  // map_weights (WenoLimiter.h:12-17)
     const double d = i == 1 ? kD1 : (i == 3 ? kD3 : kD0);
