@@ -439,8 +439,10 @@ __device__ __forceinline__ void sweep_tile(const typename P::Args &A, const int 
         sAbort = 1;
       }
       // (generic reads of a slot, then a TMA write into it after barrier (A): ordered by
-      // the barrier. Generic writes into slots a TMA box later fills happen only in the
-      // prologue -- fenced there -- or in the last chunks, after the tile's last box.)
+      // the barrier. Within a tile, generic writes into slots that a TMA box fills later
+      // happen only in the prologue, which fences them, and the first chunk's boxes, issued
+      // before that fence, fill none of the prologue's slots. What a tile leaves behind, its
+      // last chunks' cp.async rows and halo values among it, is fenced at its end.)
     }
     if constexpr (ASYNC) {
       cp_async_wait_all();  // this thread's rows of the chunk have landed
@@ -665,6 +667,9 @@ __device__ __forceinline__ void sweep_tile(const typename P::Args &A, const int 
     if (late0) finish_first(qL, qR, F);
   }
   if constexpr (TMA) {  // every issued phase has completed (or been given up on, flagged)
+    // a persistent CTA's next tile issues its first boxes straight away: this tile's generic
+    // accesses to the ring (all of them where it had no tensor map) come before those
+    fence_proxy_async();
     __syncthreads();
     if (tid == 0) {
       // after a give-up, a last bounded wait so that no box is still landing in this
