@@ -13,6 +13,7 @@
 #include <cuda_runtime.h>
 
 #include <cstring>
+#include <type_traits>
 
 #include "awfl_internal.h"
 #include "awfl_p64.cuh"
@@ -107,13 +108,13 @@ cudaError_t launch_add_zero_fp64(double *p, int nplanes, int nx, int ny, int nz,
 // that is RN(cfl*dx / max m), and the kernel only reduces the three largest speeds; the host
 // divides. The blocks' maxima meet in acc[0..2] (bit patterns of non-negative doubles), and
 // the last block (counted in acc[3]) moves them to `result` and zeroes acc for the next call.
-// What a NaN speed hides is what the reference's comparisons hide: of the cell's directions,
-// those before it in the order x, y, z. A cell's five quotients share its density's
+// What a NaN speed hides is, in the FP64 path, what the reference's comparisons hide: of the
+// cell's directions, those before it in the order x, y, z; in the FP32 form itself alone. A cell's five quotients share its density's
 // reciprocal; a cell with a speed that is not finite is evaluated again with plain divisions,
 // whose infinities and NaN differ. Few blocks walk over the planes, so that few atomics
 // follow. awfl_cfl with its read-back, 256x256x128: 216 -> 138 us; 130x100x70: 54 -> 42.
 // ------------------------------------------------------------------------------------
-template <bool PLAIN>
+template <bool PLAIN, class T>
 __device__ __forceinline__ void cell_speeds(double r, const double (&m)[3], double rt, double (&out)[3]) {
   const Rcp<double> y = PLAIN ? rcp_known(r, 0.) : make_rcp<double>(r);
   auto over = [&](double a) { return PLAIN ? a / r : divp(a, y); };
@@ -122,13 +123,13 @@ __device__ __forceinline__ void cell_speeds(double r, const double (&m)[3], doub
 #pragma unroll
   for (int d = 0; d < 3; d++) {
     const double u = over(m[d]), a = fabs(u - cs), b = fabs(u + cs);
-    out[d] = a > b ? a : b;
+    out[d] = std::is_same<T, float>::value ? fmax(a, b) : (a > b ? a : b);
   }
 }
-static __device__ __noinline__ void cell_speeds_plain(double r, double m0, double m1, double m2, double rt, double *out) {
+template <class T> static __device__ __noinline__ void cell_speeds_plain(double r, double m0, double m1, double m2, double rt, double *out) {
   const double m[3] = {m0, m1, m2};
   double o[3];
-  cell_speeds<true>(r, m, rt, o);
+  cell_speeds<true, T>(r, m, rt, o);
   for (int d = 0; d < 3; d++) out[d] = o[d];
 }
 
@@ -145,10 +146,11 @@ __global__ void __launch_bounds__(kCellThreads) cfl_kernel(const T *state, const
       const double r = (double)p[0] + dens_c[hs + k], rt = (double)p[4 * sv] + denstheta_c[hs + k];
       const double m[3] = {(double)p[sv], (double)p[2 * sv], (double)p[3 * sv]};
       double v[3];
-      cell_speeds<false>(r, m, rt, v);
-      if (!(v[0] + v[1] + v[2] < 1e300)) cell_speeds_plain(r, m[0], m[1], m[2], rt, v);
-      if (v[2] == v[2]) {
-        if (v[1] == v[1] && v[0] > best[0]) best[0] = v[0];
+      cell_speeds<false, T>(r, m, rt, v);
+      if (!(v[0] + v[1] + v[2] < 1e300)) cell_speeds_plain<T>(r, m[0], m[1], m[2], rt, v);
+      const bool all = std::is_same<T, float>::value;
+      if (all || v[2] == v[2]) {
+        if ((all || v[1] == v[1]) && v[0] > best[0]) best[0] = v[0];
         if (v[1] > best[1]) best[1] = v[1];
         if (v[2] > best[2]) best[2] = v[2];
       }
