@@ -97,17 +97,18 @@ template <class Sc> __device__ __forceinline__ Sc divr(const Sc &a, const Rcp<Sc
 __device__ __forceinline__ double divr(const double &a, const Rcp<double> &r) { return div_markstein(a, r.b, r.y); }
 // The divisions of transported tracer values, correctly rounded for every dividend: nonzero
 // ones below 2^-900 in magnitude (where the quotient or the remainder could leave the normal
-// range, as values that decay towards zero can) take the IEEE division itself; a zero
+// range, as values that decay towards zero can) and those from 2^900 on (infinities among
+// them, of which the remainder would make a NaN) take the IEEE division itself; a zero
 // dividend stays on the short path, whose quotient is IEEE's signed zero
 // (the test on the bit pattern, off the FP64 pipe)
-__device__ __forceinline__ bool is_tiny(double a) {
+__device__ __forceinline__ bool is_extreme(double a) {
   const unsigned h = (unsigned)__double2hiint(a) & 0x7fffffffu;
-  return h < ((1023u - 900u) << 20) && (h | (unsigned)__double2loint(a)) != 0;
+  return h - ((1023u - 900u) << 20) >= (1800u << 20) && (h | (unsigned)__double2loint(a)) != 0;
 }
 // for r.b > 0, and for a divisor b known on the host as 1/b = h + l
-__device__ __forceinline__ double divp_any(double a, const Rcp<double> &r) { return is_tiny(a) ? a / r.b : divp(a, r); }
+__device__ __forceinline__ double divp_any(double a, const Rcp<double> &r) { return is_extreme(a) ? a / r.b : divp(a, r); }
 __device__ __forceinline__ double div_known_any(double a, double b, double h, double l) {
-  return is_tiny(a) ? a / b : div_known(a, h, l);
+  return is_extreme(a) ? a / b : div_known(a, h, l);
 }
 // any scalar divided by a double divisor with a known reciprocal
 template <class Sc> __device__ __forceinline__ Sc divd(const Sc &a, const Rcp<double> &r) { return a / r.b; }
@@ -132,7 +133,7 @@ __device__ __forceinline__ double divk(const double &a, int k) {
 __device__ __forceinline__ double divk_any(double a, int k) {
   if (k == 1) return a;
   if ((k & (k - 1)) == 0) return a * (1.0 / k);
-  return is_tiny(a) ? a / k : divk(a, k);
+  return is_extreme(a) ? a / k : divk(a, k);
 }
 
 // the reciprocal of 2b from that of b (exact: a power-of-two scaling)

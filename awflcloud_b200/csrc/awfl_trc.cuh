@@ -229,9 +229,10 @@ __global__ void __launch_bounds__(128, AWFL_TRC_LIMIT_MINB) tracer_limit_faces_k
       Fx out = F;
       if (((T.pos >> l) & 1ull) && c >= 0) {
         const double q = *tc;
-        if (F == Fx(0)) {
+        if (F == Fx(0) && ((unsigned)__double2hiint(q) & 0x7fffffffu) < ((1023u + 100u) << 20)) {
           // a zero times the factor, whose sign is the tracer's: a tracer absent here reads no
-          // other face and divides nothing
+          // other face and divides nothing (not so an infinite one or a NaN, which the FP32
+          // form's clamped edges turn into zero fluxes: their factor makes it a NaN again)
           out = __double2hiint(q) < 0 ? -F : F;
         } else {
           const Fx Fa = ia == 0 ? F : TF[ia], Fb = ib == 0 ? F : TF[ib];

@@ -35,3 +35,32 @@ def test_fp32_rough_tracers_follow_fp64(ord_, scale):
     for l in range(2):
         a, b = t32[box][l], t64[box][l]
         assert float((a - b).norm()) <= 1e-6 * float(b.norm()), l
+
+
+@pytest.mark.parametrize("dir_", [0, 1, 2])
+@pytest.mark.parametrize("value", ["inf", "nan", "-inf"])
+def test_fp32_limited_tracer_of_one_bad_cell(dir_, value):
+    """A positive-definite tracer of zeros with one cell that is not a number: the edges it
+    touches are clamped to zero, so the fluxes are zero and the limiter's factor min(1, r) of
+    the cell decides. +inf: the factor is 1, the cell stays +inf and nothing else moves. NaN and
+    -inf: the factor makes the cell's outflow a NaN, which reaches the cell and the one
+    downwind of it."""
+    n = (16, 12, 10)
+    c = capi.Context(*n, bc=("periodic",) * 3, precision=capi.FP32)
+    s = c.new_state()
+    s.zero_()
+    s[1 + dir_] = 20.0  # momentum along the split, everywhere
+    h = c.hs
+    at = [4, 5, 6]  # k, j, i
+    t = c.new_tracers(1)
+    t.zero_()
+    t[(0,) + tuple(h + x for x in at)] = float(value)
+    c.split_tracers(s, t, 0.1, dir_, pos=[1])
+    got = t[0, h:-h, h:-h, h:-h].cpu()
+    want = torch.zeros_like(got)
+    want[tuple(at)] = float("inf") if value == "inf" else float("nan")
+    if value != "inf":
+        at[2 - dir_] += 1
+        want[tuple(at)] = float("nan")
+    assert torch.equal(got.isnan(), want.isnan())
+    assert torch.equal(got.nan_to_num(nan=0.0, posinf=1.0), want.nan_to_num(nan=0.0, posinf=1.0))
