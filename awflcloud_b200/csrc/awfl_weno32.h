@@ -61,10 +61,15 @@ template <class T> __device__ __forceinline__ void weno_gll5(const T (&u)[5], T 
 // agree on their four shared cells, so they differ by a fifth difference D_j of six cells
 // times a fixed polynomial (w9: P_3 - P_2 = D_2 N, P_4 - P_3 = D_3 M, the mirror images on the
 // other side), and so does the bridge polynomial (four D_j, by parity in sums and differences
-// of mirror pairs). Equal to the matrix form in exact arithmetic, the weights summing to one;
-// about 260 instead of 390 FP32 instructions, and u[4] enters the values unrounded: their
-// error against FP64 is a third of the matrix form's (random, smooth and jump stencils). The
-// sweep is issue-bound: 128x128x64 step 0.608 -> 0.483 ms.
+// of mirror pairs). The outer candidates' indicators take their coefficients from their own
+// differences: two steps of D_j from P_2's lose a smooth outer candidate in a rough stencil
+// (10 instructions, 128x128x64 step 422 -> 428 us). Equal to the matrix form in exact
+// arithmetic, the weights summing to one; about 270 instead of 390 FP32 instructions, and u[4]
+// enters the values unrounded. Error against FP64 over the stencil's largest value, matrix
+// form -> this one, root mean square and 99.9% quantile: random 6.0e-8 -> 3.4e-8 and 2.9e-7 ->
+// 2.4e-7, smooth 7.2e-8 -> 2.5e-8 and 2.8e-7 -> 8.6e-8, jump 7.6e-8 -> 2.9e-8 and 3.3e-7 ->
+// 1.2e-7; the largest of 4 million random stencils 8.5e-7 -> 9.2e-7. The sweep is issue-bound:
+// 128x128x64 step 0.608 -> 0.483 ms when the matrices went.
 template <class T> __device__ __forceinline__ void weno_gll9(const T (&u)[9], T (&out)[5]) {
   using namespace w9;
   T d1[8], d2[7], d3[6], d4[5], D[4];
@@ -93,10 +98,14 @@ template <class T> __device__ __forceinline__ void weno_gll9(const T (&u)[9], T 
   for (int i = 1; i < 4; i++) {
     const float sg = i % 2 ? 1.f : -1.f;
     a[3][i] = fmaT((float)n.c[i], D[2], a[2][i]);
-    a[4][i] = fmaT((float)m.c[i], D[3], a[3][i]);
     a[1][i] = fmaT(sg * (float)n.c[i], D[1], a[2][i]);
-    a[0][i] = fmaT(sg * (float)m.c[i], D[0], a[1][i]);
   }
+  a[4][1] = fmaT((float)(-3. / 16), d4[4], fmaT((float)(7. / 24), d3[4], fmaT(-.5f, d2[4], d1[4])));
+  a[4][2] = fmaT((float)(7. / 16), d4[4], .5f * (d2[4] - d3[4]));
+  a[4][3] = fmaT(-.25f, d4[4], (float)(1. / 6) * d3[4]);
+  a[0][1] = fmaT((float)(3. / 16), d4[0], fmaT((float)(7. / 24), d3[1], fmaT(.5f, d2[2], d1[3])));
+  a[0][2] = fmaT((float)(7. / 16), d4[0], .5f * (d2[2] + d3[1]));
+  a[0][3] = fmaT(.25f, d4[0], (float)(1. / 6) * d3[1]);
   // the bridge polynomial's
   const T se = D[2] - D[1], so = D[2] + D[1], te = D[3] - D[0], to = D[3] + D[0];
   T h[9];

@@ -40,3 +40,8 @@ def check(tmp_path_factory):
 @pytest.mark.parametrize("ord_", [5, 9])
 def test_reconstruction_follows_fp64_at_every_scale(check, ord_):
     check("scales%d" % ord_)
+
+
+@pytest.mark.parametrize("ord_", [5, 9])
+def test_errors_no_larger_than_the_matrix_form(check, ord_):
+    check("errors%d" % ord_)
