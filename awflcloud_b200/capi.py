@@ -75,6 +75,7 @@ _SIGS = {
     "awfl_step": (_I, [_VP, _VP, _D, _VP]),
     "awfl_step_tlm": (_I, [_VP, _VP, _D, _VP]),
     "awfl_create_slab": (_I, [ctypes.POINTER(AwflConfig), _I, _I, _I, ctypes.POINTER(_VP)]),
+    "awfl_sweep_shape": (_I, [_VP, _VP, _I, _I, ctypes.POINTER(_I)]),
     "awfl_slab_info": (_I, [_VP] + [ctypes.POINTER(_I)] * 4 + [ctypes.POINTER(_L)]),
     "awfl_slab_pack": (_I, [_VP, _VP, _VP, _VP]),
     "awfl_split_slab": (_I, [_VP, _VP, _VP, _D, _VP]),
@@ -207,6 +208,12 @@ class Context:
     @staticmethod
     def _local_nx(nx, nslabs, slab):
         return nx // nslabs + (1 if slab < nx % nslabs else 0)
+
+    def sweep_shape(self, d, form=0, state=None):
+        """(cells at a time, lines per CTA, rows by TMA) of a sweep along d (awfl_sweep_shape)."""
+        v = (_I * 3)()
+        self._check(self.L.awfl_sweep_shape(self.h, None if state is None else state.data_ptr(), form, d, v))
+        return v[0], v[1], bool(v[2])
 
     def slab_info(self):
         v = [_I() for _ in range(4)]

@@ -95,6 +95,7 @@ template <int ORD, int DIR> struct PolicyShapes<P64Rec, ORD, DIR> : RecordShapes
 cudaError_t launch_sweep_rec(int ord, int dir, const SweepArgs &A, cudaStream_t st) {
   return launch_sweep_any<P64Rec>(ord, dir, A, st);
 }
+SweepChoice sweep_choice_rec(int ord, int dir, const SweepArgs &A) { return sweep_choice_any<P64Rec>(ord, dir, A); }
 
 cudaError_t upload_tables_adj(int ord, const void *tab, size_t bytes) {
   if (ord == 5) return cudaMemcpyToSymbol(c_tab5, tab, bytes);

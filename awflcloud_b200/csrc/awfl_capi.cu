@@ -863,6 +863,26 @@ int awfl_create_slab(const awfl_config *global, int nslabs, int slab, int device
   return AWFL_OK;
 }
 
+int awfl_sweep_shape(awfl_ctx *c, const void *d_state, int form, int dir, int shape[3]) {
+  if (!c || !shape) return AWFL_ERR_ARG;
+  if (dir < 0 || dir > 2) return fail(c, AWFL_ERR_ARG, "dir must be 0, 1 or 2");
+  if (form < 0 || form > 2 || (form == 2 && fp32(c)))
+    return fail(c, AWFL_ERR_ARG, "awfl_sweep_shape: form must be 0, 1 or (FP64) 2");
+  SweepChoice s;
+  if (fp32(c)) {
+    const SweepArgs32 A = sweep_args32(c, const_cast<void *>(d_state), nullptr, 0.0, dir, MODE_APPLY);
+    s = form == 0 ? sweep_choice_fp32(c->cfg.ord, dir, A) : sweep_choice_tracers32(c->cfg.ord, dir, A);
+  } else {
+    const SweepArgs A = sweep_args(c, const_cast<void *>(d_state), nullptr, 0.0, dir, MODE_APPLY);
+    s = form == 0 ? sweep_choice_fp64(c->cfg.ord, dir, A)
+                  : (form == 1 ? sweep_choice_tracers(c->cfg.ord, dir, A) : sweep_choice_rec(c->cfg.ord, dir, A));
+  }
+  shape[0] = s.C;
+  shape[1] = s.W;
+  shape[2] = d_state ? s.tma : 0;
+  return AWFL_OK;
+}
+
 int awfl_slab_info(const awfl_ctx *c, int *nslabs, int *slab, int *xoff, int *nx_global, long *halo_elems) {
   if (!c) return AWFL_ERR_ARG;
   if (nslabs) *nslabs = c->nslabs;

@@ -66,6 +66,7 @@ bool encode_state_map32(TmaMap *m, const float *state, int xe, int ye, int ze, c
 cudaError_t launch_sweep_fp32(int ord, int dir, const SweepArgs32 &A, cudaStream_t st) {
   return launch_sweep_any<P32>(ord, dir, A, st);
 }
+SweepChoice sweep_choice_fp32(int ord, int dir, const SweepArgs32 &A) { return sweep_choice_any<P32>(ord, dir, A); }
 
 cudaError_t upload_tables_fp32(int ord, const double *recon, const double *c2g, const double *s2g,
                                const double *deriv, const double *idl, double sigma, const double *wts) {

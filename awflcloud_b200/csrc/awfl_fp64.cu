@@ -23,6 +23,7 @@ namespace awfl {
 cudaError_t launch_sweep_fp64(int ord, int dir, const SweepArgs &A, cudaStream_t st) {
   return launch_sweep_any<P64>(ord, dir, A, st);
 }
+SweepChoice sweep_choice_fp64(int ord, int dir, const SweepArgs &A) { return sweep_choice_any<P64>(ord, dir, A); }
 
 
 

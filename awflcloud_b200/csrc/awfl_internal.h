@@ -146,6 +146,16 @@ struct InitLaunch {
 // FP32 form (awfl_fp32.cu)
 struct SweepArgs32;
 cudaError_t launch_sweep_fp32(int ord, int dir, const SweepArgs32 &A, cudaStream_t st);
+// The tile shape that a sweep's launch takes (chunk C x lines W) and its staging, for the plain
+// sweeps, the tracer splits' and the adjoint's recording ones.
+struct SweepChoice {
+  int C, W, tma;
+};
+SweepChoice sweep_choice_fp32(int ord, int dir, const SweepArgs32 &A);
+SweepChoice sweep_choice_tracers32(int ord, int dir, const SweepArgs32 &A);
+SweepChoice sweep_choice_fp64(int ord, int dir, const SweepArgs &A);
+SweepChoice sweep_choice_tracers(int ord, int dir, const SweepArgs &A);
+SweepChoice sweep_choice_rec(int ord, int dir, const SweepArgs &A);
 cudaError_t launch_apply_fp32(float *state, float *comp, const float *tend, float dt, int nx, int ny, int nz, int hs,
                               int nsm, cudaStream_t st);
 cudaError_t upload_tables_fp32(int ord, const double *recon, const double *c2g, const double *s2g,

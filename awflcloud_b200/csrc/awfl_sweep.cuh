@@ -719,6 +719,9 @@ template <class P, int ORD, int DIR> struct PolicyShape : SweepShape<ORD, DIR> {
 
 // Policies with wider elements (P::kWdiv > 1) use fewer lines per CTA to stay within the
 // 48 KB of static shared memory.
+template <class P, int ORD, int DIR, int C> constexpr bool stages_by_tma() {
+  return P::kTmaRing && ORD == 5 && DIR != 2 && C == PolicyShape<P, ORD, DIR>::C;
+}
 template <class P, int ORD, int DIR, int C, int W>
 cudaError_t launch_sweep_shape(const typename P::Args &A, cudaStream_t st) {
   dim3 grid;
@@ -729,7 +732,7 @@ cudaError_t launch_sweep_shape(const typename P::Args &A, cudaStream_t st) {
   // the x split of a slab with neighbouring slabs' columns: the SLAB instantiation
   bool slab = false;
   if constexpr (DIR == 0 && P::kSlab && base) slab = A.xh[0] != nullptr || A.xh[1] != nullptr;
-  if constexpr (P::kTmaRing && ORD == 5 && DIR != 2 && base) {
+  if constexpr (stages_by_tma<P, ORD, DIR, C>()) {
     // the policy encodes this launch's tensor map (box = one chunk of one variable); a
     // layout TMA cannot address (alignment) leaves tma off and the cp.async path runs. TMA only
     // where it is the faster: the x and y shapes of large grids (FP32 256x256x128, us, TMA
@@ -775,16 +778,16 @@ inline double sweep_cost(int C, int L, long tiles, int nsm, bool ends, int slots
 // 97x61x45 39.4 49.6 41.5 -> 33.4 25.2 31.2, 400x1x200 120 - 129 -> 18.6 - 18.7.
 template <class P, int ORD, int DIR, class = void> struct PolicyShapes { static constexpr int n = 0; };
 
-template <class P, int ORD, int DIR>
-cudaError_t launch_sweep_t(const typename P::Args &A, cudaStream_t st) {
+// the index in PolicyShapes of the shape that a sweep takes, -1 for PolicyShape
+template <class P, int ORD, int DIR> int sweep_shape(const typename P::Args &A) {
   using B = PolicyShape<P, ORD, DIR>;
   constexpr int BW = B::W / P::kWdiv > 0 ? B::W / P::kWdiv : 1;
   using S = PolicyShapes<P, ORD, DIR>;
+  int best = -1;
   if constexpr (S::n > 0) {
     const int L = DIR == 0 ? A.nx : (DIR == 1 ? A.ny : A.nz);
     const int across = DIR == 0 ? A.ny : A.nx;  // lines of one plane, W to a tile
     const long planes = DIR == 2 ? A.ny : A.nz;
-    int best = -1;
     constexpr int slots = ORD == 5 ? 4 : (P::min_blocks(ORD) > 2 ? P::min_blocks(ORD) : 2);
     constexpr double share = ORD == 5 ? 0.4 : 0.2;
     double cost = 0.95 * P::base_factor(A) * sweep_cost(B::C, L, (across + BW - 1) / BW * planes, A.nsm, false, slots, share);
@@ -795,6 +798,17 @@ cudaError_t launch_sweep_t(const typename P::Args &A, cudaStream_t st) {
     if constexpr (DIR == 0 && P::kSlab) {
       if (A.xh[0] != nullptr || A.xh[1] != nullptr) best = -1;
     }
+  }
+  return best;
+}
+
+template <class P, int ORD, int DIR>
+cudaError_t launch_sweep_t(const typename P::Args &A, cudaStream_t st) {
+  using B = PolicyShape<P, ORD, DIR>;
+  constexpr int BW = B::W / P::kWdiv > 0 ? B::W / P::kWdiv : 1;
+  using S = PolicyShapes<P, ORD, DIR>;
+  if constexpr (S::n > 0) {
+    const int best = sweep_shape<P, ORD, DIR>(A);
     if constexpr (S::n > 0) if (best == 0) return launch_sweep_shape<P, ORD, DIR, S::C[0], S::W[0]>(A, st);
     if constexpr (S::n > 1) if (best == 1) return launch_sweep_shape<P, ORD, DIR, S::C[1], S::W[1]>(A, st);
     if constexpr (S::n > 2) if (best == 2) return launch_sweep_shape<P, ORD, DIR, S::C[2], S::W[2]>(A, st);
@@ -814,6 +828,21 @@ cudaError_t launch_sweep_any(int ord, int dir, const typename P::Args &A, cudaSt
   if (dir == 0) return launch_sweep_t<P, 9, 0>(A, st);
   if (dir == 1) return launch_sweep_t<P, 9, 1>(A, st);
   return launch_sweep_t<P, 9, 2>(A, st);
+}
+
+// What a launch with these arguments takes (diagnostics): C, W, and whether its rows come by TMA.
+template <class P, int ORD, int DIR> SweepChoice sweep_choice_t(typename P::Args A) {
+  using B = PolicyShape<P, ORD, DIR>;
+  using S = PolicyShapes<P, ORD, DIR>;
+  const int i = sweep_shape<P, ORD, DIR>(A);
+  if constexpr (S::n > 0) if (i >= 0) return SweepChoice{S::C[i], S::W[i], 0};
+  SweepChoice c{B::C, B::W / P::kWdiv > 0 ? B::W / P::kWdiv : 1, 0};
+  if constexpr (stages_by_tma<P, ORD, DIR, B::C>()) c.tma = P::prepare_tma(A, ORD, DIR, c.C, c.W);
+  return c;
+}
+template <class P> SweepChoice sweep_choice_any(int ord, int dir, const typename P::Args &A) {
+  if (ord == 5) return dir == 0 ? sweep_choice_t<P, 5, 0>(A) : (dir == 1 ? sweep_choice_t<P, 5, 1>(A) : sweep_choice_t<P, 5, 2>(A));
+  return dir == 0 ? sweep_choice_t<P, 9, 0>(A) : (dir == 1 ? sweep_choice_t<P, 9, 1>(A) : sweep_choice_t<P, 9, 2>(A));
 }
 
 }  // namespace awfl

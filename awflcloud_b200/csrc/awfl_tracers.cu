@@ -303,6 +303,8 @@ cudaError_t run(const TracerArgs &T, int io, cudaStream_t st) {
 
 }  // namespace
 
+SweepChoice sweep_choice_tracers(int ord, int dir, const SweepArgs &A) { return sweep_choice_any<P64Trc>(ord, dir, A); }
+
 cudaError_t launch_split_tracers(int ord, int dir, const SweepArgs &Ain, double *tracers, int ntr,
                                  unsigned long long pos, double *scratch, int io, cudaStream_t st) {
   const int ng = ord == 5 ? 3 : 5;

@@ -331,6 +331,8 @@ cudaError_t run32(const TracerArgs32 &T, int io, cudaStream_t st) {
 
 }  // namespace
 
+SweepChoice sweep_choice_tracers32(int ord, int dir, const SweepArgs32 &A) { return sweep_choice_any<P32Trc>(ord, dir, A); }
+
 cudaError_t launch_split_tracers32(int ord, int dir, const SweepArgs32 &Ain, const double *dens_c, double dt,
                                    double dxd, double *tracers, int ntr, unsigned long long pos, float *scratch,
                                    int io, cudaStream_t st) {

@@ -235,6 +235,13 @@ int awfl_slab_info(const awfl_ctx *ctx, int *nslabs, int *slab, int *xoff, int *
 int awfl_slab_pack(awfl_ctx *ctx, const void *d_state, void *d_send, void *stream);
 int awfl_split_slab(awfl_ctx *ctx, void *d_state, const void *d_recv, double dt, void *stream);
 
+/* Diagnostics: the tile of one sweep launch along dir as this context would take it: shape[0]
+ * cells of a line at a time, shape[1] lines per CTA, shape[2] whether its rows come by TMA (0
+ * for a NULL d_state; otherwise d_state's alignment decides with the rest). form: 0 the plain
+ * split, 1 the tracer split's, 2 the adjoint's recording sweep (FP64). Launches nothing; a
+ * host-only context answers for 148 SMs. */
+int awfl_sweep_shape(awfl_ctx *ctx, const void *d_state, int form, int dir, int shape[3]);
+
 /* Tangent-linear time step (FP64 contexts): d_state_tangent holds two FP64 state planes,
  * the state then a perturbation direction. The state advances exactly like awfl_step
  * (bit-identical) and the second plane becomes the derivative of the new state along the
