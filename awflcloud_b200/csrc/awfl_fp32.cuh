@@ -476,9 +476,9 @@ struct P32 {
   // 0.433 at three
   static constexpr int min_blocks(int ord) { return ord == 5 ? 5 : 3; }
   using Args = SweepArgs32;
-  // rows that TMA cannot address (16-byte pitch) come by cp.async: 107 instead of about 85 us
-  // for the x split of 130x100x70
-  static double base_factor(const Args &A) { return A.nx % 4 ? 1.25 : 1.0; }
+  // where the base shape's rows come by TMA (`tma`), those that it cannot address (16-byte
+  // pitch) come by cp.async: 107 instead of about 85 us for the x split of 130x100x70
+  static double base_factor(const Args &A, bool tma) { return tma && A.nx % 4 ? 1.25 : 1.0; }
   // the Kahan compensations of the cell's five variables, loaded before the reconstruction
   struct Aux {
     float c[5];
@@ -521,6 +521,7 @@ struct P32 {
 // y 8 x 16, z 4 x 32 (y/z: a warp = 32/C lines x C positions). Measured at 256x256x128, five
 // CTAs per SM, us per split: x 8x16 374, 16x8 372, 8x8 (64 threads) 425; y 8x16 385, 4x32
 // 401, 8x8 385, 4x16 418; z 4x32 388, 8x16 408, 4x64 511, 4x16 438.
+// (z at 254x256x128, whose rows TMA could not address: 385, 8x16 428.)
 template <> struct PolicyShape<P32, 5, 0> { static constexpr int C = 8, W = 16; };
 template <> struct PolicyShape<P32, 5, 1> { static constexpr int C = 8, W = 16; };
 // Ord 9, three CTAs of 128 threads (128x128x64, us): x 32 x 4 138, 8 x 16 154; y 16 x 8 141,

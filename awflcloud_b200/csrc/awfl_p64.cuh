@@ -26,7 +26,7 @@ struct P64 {
 #endif
   static constexpr int min_blocks(int ord) { return ord == 5 ? AWFL_P64_MIN_BLOCKS_ORD5 : 1; }
   using Args = SweepArgs;
-  static double base_factor(const Args &) { return 1.0; }
+  static double base_factor(const Args &, bool) { return 1.0; }
   struct Aux {};
   static __device__ __forceinline__ void load_aux(const Args &, long, long, Aux &) {}
 

@@ -48,7 +48,7 @@
 //                                          global memory for ensembles)
 //   min_blocks(ORD)                        CTAs per SM the register budget must allow
 //   kSlab                                  the policy runs x splits of slabs (A.xh)
-//   base_factor(A)                         (host) what keeps PolicyShape from its usual speed
+//   base_factor(A, tma)                    (host) what keeps PolicyShape from its usual speed
 //   load(A, gidx) / store(A, gidx, x)      state element access (halo writes)
 //   store_tend(A, tidx, x)                 tendency output (MODE_TEND)
 #pragma once
@@ -790,7 +790,8 @@ template <class P, int ORD, int DIR> int sweep_shape(const typename P::Args &A) 
     const long planes = DIR == 2 ? A.ny : A.nz;
     constexpr int slots = ORD == 5 ? 4 : (P::min_blocks(ORD) > 2 ? P::min_blocks(ORD) : 2);
     constexpr double share = ORD == 5 ? 0.4 : 0.2;
-    double cost = 0.95 * P::base_factor(A) * sweep_cost(B::C, L, (across + BW - 1) / BW * planes, A.nsm, false, slots, share);
+    double cost = 0.95 * P::base_factor(A, stages_by_tma<P, ORD, DIR, B::C>()) *
+                  sweep_cost(B::C, L, (across + BW - 1) / BW * planes, A.nsm, false, slots, share);
     for (int i = 0; i < S::n; i++) {
       const double c = S::factor[i] * sweep_cost(S::C[i], L, (across + S::W[i] - 1) / S::W[i] * planes, A.nsm, true, slots, share);
       if (c < cost) { best = i; cost = c; }

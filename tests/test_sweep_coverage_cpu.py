@@ -66,3 +66,14 @@ def test_query_refuses_what_no_sweep_takes():
     for d, form in ((3, 0), (-1, 0), (0, 3), (0, 2)):  # the adjoint is FP64's
         with pytest.raises(Exception, match="dir must be|form must be"):
             c.sweep_shape(d, form)
+
+
+@pytest.mark.parametrize("ord_,dirs", [(5, (2,)), (9, (0, 1, 2))])
+@pytest.mark.parametrize("n", [(254, 256, 128), (250, 250, 128), (1022, 64, 64)])
+def test_rows_that_tma_cannot_address_matter_only_where_tma_is_used(ord_, dirs, n):
+    """The FP32 z sweep and every ord-9 one stage by cp.async whatever the row pitch: they take
+    the shape of the next wider grid whose rows are a multiple of 16 bytes."""
+    narrow = capi.Context(*n, ord_=ord_, precision=capi.FP32, device=-1)
+    wide = capi.Context(n[0] + 2, *n[1:], ord_=ord_, precision=capi.FP32, device=-1)
+    for d in dirs:
+        assert narrow.sweep_shape(d) == wide.sweep_shape(d), d

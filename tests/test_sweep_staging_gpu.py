@@ -18,7 +18,7 @@ BUBBLE = dict(kind=capi.INIT_BUBBLE, noise_amp=0.01)
 FP64 = {9: [((200, 18, 18), PPW, {1: (8, 16), 2: (8, 16)})]}
 FP32 = {5: [((92, 107, 50), PPW, {0: (8, 16), 1: (8, 16), 2: (4, 32)}), ((52, 10, 130), PPP, {1: (4, 32)}),
             ((17, 28, 130), WWW, {0: (4, 32)})],
-        9: [((43, 9, 41), PPP, {1: (8, 16)}), ((44, 83, 9), PPW, {2: (8, 16)})]}
+        9: [((200, 18, 18), PPP, {1: (8, 16)}), ((44, 83, 9), PPW, {2: (8, 16)})]}
 RECORD = [((9, 9, 51), PPP, {0: (16, 8), 2: (128, 1)}), ((135, 45, 9), PPW, {2: (8, 16)}),
           ((9, 58, 58), WWW, {0: (8, 16), 1: (128, 1)}), ((200, 18, 18), PPP, {0: (128, 1), 1: (8, 16)}),
           ((9, 10, 9), PPP, {0: (32, 4), 1: (16, 8), 2: (16, 8)}), ((12, 18, 25), PPW, {1: (32, 4), 2: (32, 4)})]
