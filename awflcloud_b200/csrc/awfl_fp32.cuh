@@ -33,6 +33,7 @@
 #include "awfl_internal.h"
 #include "awfl_fp32_args.h"
 #include "awfl_pow.cuh"
+#include "awfl_recip.h"
 #include "awfl_sweep.cuh"
 
 namespace awfl {
@@ -206,9 +207,6 @@ template <int NG> __device__ __forceinline__ Pts<NG> same(float x) {
 // centre; at ord 5 it is {-3 4 -1; -1 0 1; 1 -4 3})
 template <int ORD> __device__ __forceinline__ Pts<OrdTraits<ORD>::NGLL> deriv32(const Pts<OrdTraits<ORD>::NGLL> &x, float sc) {
   constexpr int NG = OrdTraits<ORD>::NGLL;
-  constexpr double kD[3][5] = {{-10, 13.51300497744848, -16. / 3, 2.8203283558848535, -1},
-                               {-2.4819805060619657, 0, 3.4914862437758787, -1.5275252316519454, 0.5180194939380343},
-                               {.75, -2.6731691553909065, 0, 2.6731691553909065, -.75}};
   Pts<NG> r;
   if constexpr (ORD == 5) {
     const float x0 = x.get(0), x1 = x.c, x2 = x.get(2);
@@ -218,11 +216,12 @@ template <int ORD> __device__ __forceinline__ Pts<OrdTraits<ORD>::NGLL> deriv32(
   } else {
     // the rows of mirror points are each other's reverse negated: lane y takes the same
     // coefficients on the reversed values, and -sc (128x128x64 step 0.483 -> 0.476 ms)
+    constexpr w9::Deriv kD = w9::kD;
     auto rev = [](F2 a) { return F2(a.v.y, a.v.x); };
     const F2 p0 = x.p[0], p1 = x.p[1], m0 = rev(p0), m1 = rev(p1), cc = F2(x.c), pm = F2(sc, -sc);
-    r.p[0] = pm * fmaT((float)kD[0][0], p0, fmaT((float)kD[0][1], p1, fmaT((float)kD[0][2], cc, fmaT((float)kD[0][3], m1, (float)kD[0][4] * m0))));
-    r.p[1] = pm * fmaT((float)kD[1][0], p0, fmaT((float)kD[1][2], cc, fmaT((float)kD[1][3], m1, (float)kD[1][4] * m0)));
-    const F2 h = fmaT((float)kD[2][0], p0, (float)kD[2][1] * p1);
+    r.p[0] = pm * fmaT((float)kD.d[0][0], p0, fmaT((float)kD.d[0][1], p1, fmaT((float)kD.d[0][2], cc, fmaT((float)kD.d[0][3], m1, (float)kD.d[0][4] * m0))));
+    r.p[1] = pm * fmaT((float)kD.d[1][0], p0, fmaT((float)kD.d[1][2], cc, fmaT((float)kD.d[1][3], m1, (float)kD.d[1][4] * m0)));
+    const F2 h = fmaT((float)kD.d[2][0], p0, (float)kD.d[2][1] * p1);
     r.c = sc * (h.v.x - h.v.y);
     return r;
   }
@@ -553,28 +552,14 @@ static inline cudaError_t upload_tables32_here(int ord, const double *recon, con
     for (int i = 0; i < g * g; i++) t.deriv[i] = (float)deriv[i];
     for (int i = 0; i < g; i++) t.wts[i] = (float)wts[i];
   };
-  // what the FP32 forms take as compile-time constants, against the tables they come from
-  auto near = [](double a, double b) { return fabs(a - b) <= 1e-12 * fmax(1.0, fabs(b)); };
-  bool ok = near(deriv[(ord == 5 ? 1 : 2) * (ord == 5 ? 3 : 5) + (ord == 5 ? 1 : 2)], 0.0);
+  if (!host::fp32_forms_match(ord, recon, c2g, deriv, idl, sigma)) return cudaErrorInvalidValue;
   if (ord == 5) {
     Tables32<5> t;
     fill(t, 5, 3);
-    ok = ok && near(sigma, w5::kSigma);
-    for (int i = 0; i < 4; i++) ok = ok && near(idl[i], i == 1 ? w5::kD1 : (i == 3 ? w5::kD3 : w5::kD0));
-    if (!ok) return cudaErrorInvalidValue;
     return cudaMemcpyToSymbol(c32_tab5, &t, sizeof t);
   }
   Tables32<9> t;
   fill(t, 9, 5);
-  ok = ok && near(sigma, w9::kSigma) && near(c2g[1 * 5 + 3], w9::kX1) && near(c2g[1 * 5 + 4], 0.5);
-  for (int i = 0; i < 6; i++) ok = ok && near(idl[i], w9::ideal(i));
-  for (int i = 0; i < 9; i++) {
-    // u = 1 in cell 7 (D_2 = 1, D_3 = -5), then in cell 8 (D_3 = 1); P_2 = 0 for both
-    if (i < 5) ok = ok && near(recon[(3 * 9 + 4) * 9 + i], w9::kN.c[i]) && near(recon[(4 * 9 + 4) * 9 + i], w9::kM.c[i]);
-    ok = ok && near(recon[(5 * 9 + 7) * 9 + i], w9::kFa.c[i] - 5 * w9::kFb.c[i]) &&
-         near(recon[(5 * 9 + 8) * 9 + i], w9::kFb.c[i]);
-  }
-  if (!ok) return cudaErrorInvalidValue;
   return cudaMemcpyToSymbol(c32_tab9, &t, sizeof t);
 }
 

@@ -73,6 +73,14 @@ constexpr Poly bridge(const Poly &f, double d, const Poly &p) {
   for (int i = 0; i < 9; i++) r.c[i] = (f.c[i] - d * p.c[i]) / ideal(5);
   return r;
 }
+// d/dx at the GLL points -1/2, -kX1, 0 from the values at all five; those of the mirror points
+// are each other's reverse negated
+struct Deriv {
+  double d[3][5];
+};
+constexpr Deriv kD = {{{-10, 13.51300497744848, -16. / 3, 2.8203283558848535, -1},
+                       {-2.4819805060619657, 0, 3.4914862437758787, -1.5275252316519454, 0.5180194939380343},
+                       {.75, -2.6731691553909065, 0, 2.6731691553909065, -.75}}};
 constexpr Poly kHa = bridge(kFa, ideal(0) + ideal(1), kN), kHb = bridge(kFb, ideal(0), kM);
 }  // namespace w9
 

@@ -81,5 +81,30 @@ template <int ORD> bool complete_tables(Tables<ORD> &t) {
   return ok;
 }
 
+// What the FP32 forms (weno_gll5, weno_gll9, deriv32) hold as compile-time constants, against
+// the tables that they come from.
+inline bool fp32_forms_match(int ord, const double *recon, const double *c2g, const double *deriv, const double *idl,
+                             double sigma) {
+  auto near = [](double a, double b) { return std::fabs(a - b) <= 1e-12 * std::fmax(1.0, std::fabs(b)); };
+  if (ord == 5) {
+    static const double der[9] = {-3., -1., 1., 4., 0., -4., -1., 1., 3.};
+    bool ok = near(sigma, w5::kSigma);
+    for (int i = 0; i < 4; i++) ok = ok && near(idl[i], i == 1 ? w5::kD1 : (i == 3 ? w5::kD3 : w5::kD0));
+    for (int x = 0; x < 9; x++) ok = ok && near(deriv[x], der[x]);
+    return ok;
+  }
+  bool ok = near(sigma, w9::kSigma) && near(c2g[1 * 5 + 3], w9::kX1) && near(c2g[1 * 5 + 4], 0.5);
+  for (int i = 0; i < 6; i++) ok = ok && near(idl[i], w9::ideal(i));
+  for (int i = 0; i < 9; i++) {
+    // u = 1 in cell 7 (D_2 = 1, D_3 = -5), then in cell 8 (D_3 = 1); P_2 = 0 for both
+    if (i < 5) ok = ok && near(recon[(3 * 9 + 4) * 9 + i], w9::kN.c[i]) && near(recon[(4 * 9 + 4) * 9 + i], w9::kM.c[i]);
+    ok = ok && near(recon[(5 * 9 + 7) * 9 + i], w9::kFa.c[i] - 5 * w9::kFb.c[i]) &&
+         near(recon[(5 * 9 + 8) * 9 + i], w9::kFb.c[i]);
+  }
+  for (int s = 0; s < 5; s++)
+    for (int ii = 0; ii < 5; ii++) ok = ok && near(deriv[s * 5 + ii], ii < 3 ? w9::kD.d[ii][s] : -w9::kD.d[4 - ii][4 - s]);
+  return ok;
+}
+
 }  // namespace host
 }  // namespace awfl
