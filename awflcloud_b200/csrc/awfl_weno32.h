@@ -9,8 +9,7 @@ namespace awfl {
 // The ord-5 WENO reconstruction to the three GLL points in differences of the stencil: with
 // d_i = u[i+1]-u[i] and s_i = d[i+1]-d[i], the three parabolas are u[2] - s_i/24 + a_i x +
 // (s_i/2) x^2 and the bridge polynomial has the few coefficients of w5, where the matrix
-// form multiplies 49 entries. Equal in exact arithmetic, the weights summing
-// to one; about 100 FP32 instructions instead of 150, and u[2] enters the values unrounded.
+// form multiplies 49 entries. Equal in exact arithmetic; about 100 FP32 instructions instead of 150, and u[2] enters the values unrounded.
 // The sweep is issue-bound: with the time series on point pairs
 // (Pts below), 1,500 -> 1,130 instructions per cell and split, 256x256x128 step 1.433 -> 1.200 ms.
 template <class T> __device__ __forceinline__ void weno_gll5(const T (&u)[5], T (&out)[3]) {
@@ -48,8 +47,11 @@ template <class T> __device__ __forceinline__ void weno_gll5(const T (&u)[5], T 
   inv = rcpT(((w[0] + w[1]) + (w[2] + w[3])) + eps);
   const T Q = fmaT(w[0], s0, fmaT(w[1], s1, w[2] * s2));
   const T P = fmaT(w[0], a0, fmaT(w[1], c, fmaT(w[2], a2, w[3] * fmaT(.25f, h3, h1))));
-  const T mid = fmaT(inv, fmaT((float)(-1. / 24), Q, w[3] * e0), u[2]);
-  const T ev = fmaT(inv, fmaT((float)(1. / 12), Q, w[3] * fmaT(.0625f, h4, fmaT(.25f, h2, e0))), u[2]);
+  // the normalised weights sum to 1 - eps*inv, which shows from differences of about 3e7 on:
+  // that is u[2]'s share (256x256x128 step 1136 -> 1140 us)
+  const T E = fmaT(-1.0e-20f, u[2], w[3] * e0);
+  const T mid = fmaT(inv, fmaT((float)(-1. / 24), Q, E), u[2]);
+  const T ev = fmaT(inv, fmaT((float)(1. / 12), Q, fmaT(w[3], fmaT(.0625f, h4, .25f * h2), E)), u[2]);
   const T od = (.5f * inv) * P;
   out[0] = ev - od;
   out[1] = mid;
@@ -64,7 +66,7 @@ template <class T> __device__ __forceinline__ void weno_gll5(const T (&u)[5], T 
 // of mirror pairs). The outer candidates' indicators take their coefficients from their own
 // differences: two steps of D_j from P_2's lose a smooth outer candidate in a rough stencil
 // (10 instructions, 128x128x64 step 422 -> 428 us). Equal to the matrix form in exact
-// arithmetic, the weights summing to one; about 270 instead of 390 FP32 instructions, and u[4]
+// arithmetic; about 280 instead of 390 FP32 instructions, and u[4]
 // enters the values unrounded. Error against FP64 over the stencil's largest value, matrix
 // form -> this one, root mean square and 99.9% quantile: random 6.0e-8 -> 3.4e-8 and 2.9e-7 ->
 // 2.4e-7, smooth 7.2e-8 -> 2.5e-8 and 2.8e-7 -> 8.6e-8, jump 7.6e-8 -> 2.9e-8 and 3.3e-7 ->
@@ -153,22 +155,27 @@ template <class T> __device__ __forceinline__ void weno_gll9(const T (&u)[9], T 
   // sum of the weights times (P_i - P_2) and (bridge - P_2), even and odd parts
   const T x2 = ((w[3] + w[4]) * inv) * D[2], x1 = ((w[0] + w[1]) * inv) * D[1];
   const T x3 = (w[4] * inv) * D[3], x0 = (w[0] * inv) * D[0], wh = w[5] * inv;
+  // the normalised weights sum to 1 - eps*inv, as at ord 5: P_2's share (428 -> 431 us)
+  const T lack = -1.0e-20f * inv, uc = fmaT(lack, u[4], u[4]), pc = fmaT(lack, p0, p0);
+  T ac[5];
+#pragma unroll
+  for (int i = 1; i < 5; i++) ac[i] = fmaT(lack, a[2][i], a[2][i]);
   const T ne = x2 - x1, no = x2 + x1, me = x3 - x0, mo = x3 + x0;
   const T ae = wh * se, ao = wh * so, be = wh * te, bo = wh * to;
   auto even = [&](double x) {
-    T r = fmaT((float)n.even(x), ne, p0);
+    T r = fmaT((float)n.even(x), ne, pc);
     r = fmaT((float)m.even(x), me, r);
     r = fmaT((float)ha.even(x), ae, r);
     return fmaT((float)hb.even(x), be, r);
   };
-  out[2] = u[4] + even(0.);
+  out[2] = uc + even(0.);
   constexpr double xs[2] = {.5, kX1};
 #pragma unroll
   for (int j = 0; j < 2; j++) {
     const double x = xs[j];
     T ev = even(x);
-    ev = u[4] + fmaT((float)(x * x), fmaT((float)(x * x), a[2][4], a[2][2]), ev);
-    T od = (float)x * fmaT((float)(x * x), a[2][3], a[2][1]);
+    ev = uc + fmaT((float)(x * x), fmaT((float)(x * x), ac[4], ac[2]), ev);
+    T od = (float)x * fmaT((float)(x * x), ac[3], ac[1]);
     od = fmaT((float)n.odd(x), no, od);
     od = fmaT((float)m.odd(x), mo, od);
     od = fmaT((float)ha.odd(x), ao, od);

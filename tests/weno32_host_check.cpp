@@ -129,7 +129,8 @@ template <int ORD> static long check_errors(long n, const Tables<ORD> &T) {
   const Matrices<ORD> M(T);
   long bad = 0;
   for (int kind = 0; kind < 5; kind++)
-    for (double scale : {1.0, 1e3, 1e6}) {
+    for (double scale : {1.0, 1e3, 1e6, 1e9}) {
+      if (scale > 1e8 && (kind == 0 || kind == 2)) continue;  // FP32 squares of the indicators overflow
       std::mt19937_64 g(12 + kind);
       std::vector<double> e[2];
       double sq[2] = {0, 0};
