@@ -288,7 +288,7 @@ AWFL_AHD void gll5_vjp(const double (&u)[5], const double (&lout)[3], double (&l
     S1 += w0[i];
   }
   const double r1 = arcp(S1);
-  double x[4], w[4], dm[4], S2 = eps;
+  double x[4], w[4], dm[4], S2 = 0.;
   AWFL_UNROLL for (int i = 0; i < 4; i++) {
     const double d = i == 1 ? kD1 : (i == 3 ? kD3 : kD0);
     x[i] = w0[i] * r1;
@@ -297,9 +297,9 @@ AWFL_AHD void gll5_vjp(const double (&u)[5], const double (&lout)[3], double (&l
     dm[i] = ((N + x[i] * (2. * x[i] - 3. * d)) - w[i] * (1. - 2. * d)) * rD;  // d w / d x
     S2 += w[i];
   }
-  const double r2 = arcp(S2);
+  const double r2 = arcp(S2 + eps);
   AWFL_UNROLL for (int i = 0; i < 4; i++) w[i] *= r2;
-  // ---- reverse: out = (ev - od, mid, ev + od), od = P/2, mid = u[2] + w3 e0 - Q/24,
+  // ---- reverse: out = (ev - od, mid, ev + od), od = P/2, mid = S2 r2 u[2] + w3 e0 - Q/24,
   // ev = mid + Q/8 + w3 (h2/4 + h4/16), Q = sum w_i s_i, P = sum w_i a_i + w3 (h1 + h3/4)
   const double lev = lout[0] + lout[2], lmid = lout[1] + lev, lP = .5 * (lout[2] - lout[0]);
   const double lQ = .125 * lev - (1. / 24) * lmid;
@@ -314,6 +314,7 @@ AWFL_AHD void gll5_vjp(const double (&u)[5], const double (&lout)[3], double (&l
   double lh1 = w[3] * lP, lh3 = .25 * lh1, lh2 = .25 * (w[3] * lev), lh4 = .25 * lh2;
   double dot = 0.;
   AWFL_UNROLL for (int i = 0; i < 4; i++) dot += lw[i] * w[i];
+  dot -= lmid * u[2] * (eps * r2);  // the weights' sum, S2 r2, is u[2]'s share in mid
   AWFL_UNROLL for (int i = 0; i < 4; i++) lw[i] = r2 * (lw[i] - dot) * dm[i];
   dot = 0.;
   AWFL_UNROLL for (int i = 0; i < 4; i++) dot += lw[i] * x[i];
@@ -336,7 +337,7 @@ AWFL_AHD void gll5_vjp(const double (&u)[5], const double (&lout)[3], double (&l
   const double ld1 = la[0] + la[1] + ls[0] - ls[1], ld2 = la[2] + ls[1] - ls[2];
   lu[0] += ls[0];
   lu[1] -= ls[0] + ld1;
-  lu[2] += lmid + ld1 - ld2;
+  lu[2] += lmid * (S2 * r2) + ld1 - ld2;
   lu[3] += ld2 - ls[2];
   lu[4] += ls[2];
 }
