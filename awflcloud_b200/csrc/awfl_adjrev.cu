@@ -75,37 +75,36 @@ __global__ void zero_halo_kernel(double *lam, int nx, int ny, int nz, int hs) {
   }
 }
 
-static unsigned grid_for(long n, int nsm) {
-  (void)nsm;
+static unsigned grid_for(long n) {
   const long b = (n + kAdjThreads - 1) / kAdjThreads, most = 0x7fffffffL;  // one index per thread
   return (unsigned)(b < 1 ? 1 : (b < most ? b : most));
 }
 
 template <int ORD, int DIR>
-static cudaError_t split_t(const adj::SplitArgs &A, int need_edges, int nsm, cudaStream_t st) {
+static cudaError_t split_t(const adj::SplitArgs &A, int need_edges, cudaStream_t st) {
   const long n = adj::ncell_of(A), nf = adj::nface_of<DIR>(A);
-  if (need_edges) adj_edges_kernel<ORD, DIR><<<grid_for(n, nsm), kAdjThreads, 0, st>>>(A);
-  adj_face_kernel<DIR><<<grid_for(nf, nsm), kAdjThreads, 0, st>>>(A);
-  adj_cell_kernel<ORD, DIR><<<grid_for(n, nsm), kAdjThreads, 0, st>>>(A);
-  adj_weno_kernel<ORD, DIR><<<grid_for(5 * n, nsm), kAdjThreads, 0, st>>>(A);
-  adj_gather_kernel<ORD, DIR><<<grid_for(n, nsm), kAdjThreads, 0, st>>>(A);
+  if (need_edges) adj_edges_kernel<ORD, DIR><<<grid_for(n), kAdjThreads, 0, st>>>(A);
+  adj_face_kernel<DIR><<<grid_for(nf), kAdjThreads, 0, st>>>(A);
+  adj_cell_kernel<ORD, DIR><<<grid_for(n), kAdjThreads, 0, st>>>(A);
+  adj_weno_kernel<ORD, DIR><<<grid_for(5 * n), kAdjThreads, 0, st>>>(A);
+  adj_gather_kernel<ORD, DIR><<<grid_for(n), kAdjThreads, 0, st>>>(A);
   return cudaGetLastError();
 }
 
-cudaError_t launch_adjoint_split(int ord, int dir, const adj::SplitArgs &A, int need_edges, int nsm, cudaStream_t st) {
+cudaError_t launch_adjoint_split(int ord, int dir, const adj::SplitArgs &A, int need_edges, cudaStream_t st) {
   if (ord == 5) {
-    if (dir == 0) return split_t<5, 0>(A, need_edges, nsm, st);
-    if (dir == 1) return split_t<5, 1>(A, need_edges, nsm, st);
-    return split_t<5, 2>(A, need_edges, nsm, st);
+    if (dir == 0) return split_t<5, 0>(A, need_edges, st);
+    if (dir == 1) return split_t<5, 1>(A, need_edges, st);
+    return split_t<5, 2>(A, need_edges, st);
   }
-  if (dir == 0) return split_t<9, 0>(A, need_edges, nsm, st);
-  if (dir == 1) return split_t<9, 1>(A, need_edges, nsm, st);
-  return split_t<9, 2>(A, need_edges, nsm, st);
+  if (dir == 0) return split_t<9, 0>(A, need_edges, st);
+  if (dir == 1) return split_t<9, 1>(A, need_edges, st);
+  return split_t<9, 2>(A, need_edges, st);
 }
 
-cudaError_t launch_zero_halo(double *lam, int nx, int ny, int nz, int hs, int nsm, cudaStream_t st) {
+cudaError_t launch_zero_halo(double *lam, int nx, int ny, int nz, int hs, cudaStream_t st) {
   const long n = 5L * (nx + 2 * hs) * (ny + 2 * hs) * (nz + 2 * hs);
-  zero_halo_kernel<<<grid_for(n, nsm), kAdjThreads, 0, st>>>(lam, nx, ny, nz, hs);
+  zero_halo_kernel<<<grid_for(n), kAdjThreads, 0, st>>>(lam, nx, ny, nz, hs);
   return cudaGetLastError();
 }
 

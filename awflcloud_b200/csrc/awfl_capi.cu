@@ -788,10 +788,10 @@ int awfl_apply_tendencies(awfl_ctx *c, void *d_state, const void *d_tend, double
   cudaError_t e;
   if (fp32(c))
     e = launch_apply_fp32((float *)d_state, (float *)d_state + state_plane(c), (const float *)d_tend, (float)dt,
-                          c->cfg.nx, c->cfg.ny, c->cfg.nz, c->hs, c->nsm, (cudaStream_t)stream);
+                          c->cfg.nx, c->cfg.ny, c->cfg.nz, c->hs, (cudaStream_t)stream);
   else
     e = launch_apply_fp64((double *)d_state, (const double *)d_tend, dt, c->cfg.nx, c->cfg.ny, c->cfg.nz, c->hs,
-                          c->nsm, (cudaStream_t)stream);
+                          (cudaStream_t)stream);
   if (e != cudaSuccess) return cuda_fail(c, e, "apply_tendencies");
   return AWFL_OK;
 }
@@ -808,7 +808,7 @@ int awfl_split(awfl_ctx *c, void *d_state, double dt, int dir, void *stream) {
     // FP64: state += dt*0 as the reference applies them (no value changes; a -0 becomes
     // +0); the FP32 form's compensated update is left out, its state is unchanged
     if (fp32(c)) return AWFL_OK;
-    cudaError_t e = launch_add_zero_fp64((double *)d_state, 5, c->cfg.nx, c->cfg.ny, c->cfg.nz, c->hs, c->nsm,
+    cudaError_t e = launch_add_zero_fp64((double *)d_state, 5, c->cfg.nx, c->cfg.ny, c->cfg.nz, c->hs,
                                          (cudaStream_t)stream);
     return e == cudaSuccess ? AWFL_OK : cuda_fail(c, e, "split");
   }
@@ -952,10 +952,10 @@ static int split_tracers_io(awfl_ctx *c, void *d_state, double *d_tracers, int n
     // -0 becomes +0; tracers held divided between splits are -0 exactly where rho*tracer
     // is); the FP32 form leaves both unchanged
     if (fp32(c)) return AWFL_OK;
-    cudaError_t e = launch_add_zero_fp64((double *)d_state, 5, c->cfg.nx, c->cfg.ny, c->cfg.nz, c->hs, c->nsm,
+    cudaError_t e = launch_add_zero_fp64((double *)d_state, 5, c->cfg.nx, c->cfg.ny, c->cfg.nz, c->hs,
                                          (cudaStream_t)stream);
     if (e == cudaSuccess)
-      e = launch_add_zero_fp64(d_tracers, ntracers, c->cfg.nx, c->cfg.ny, c->cfg.nz, c->hs, c->nsm,
+      e = launch_add_zero_fp64(d_tracers, ntracers, c->cfg.nx, c->cfg.ny, c->cfg.nz, c->hs,
                                (cudaStream_t)stream);
     return e == cudaSuccess ? AWFL_OK : cuda_fail(c, e, "split_tracers");
   }
@@ -1084,7 +1084,7 @@ int awfl_step_adjoint(awfl_ctx *c, const void *d_state_ckpt, void *d_lambda, int
   const long ncell = (long)nx * ny * nz;
   const long nface = (long)(nx + 1) * (ny + 1) * (nz + 1);
   if (nsteps == 0) {
-    cudaError_t e = launch_zero_halo((double *)d_lambda, nx, ny, nz, c->hs, c->nsm, st);
+    cudaError_t e = launch_zero_halo((double *)d_lambda, nx, ny, nz, c->hs, st);
     return e == cudaSuccess ? AWFL_OK : cuda_fail(c, e, "adjoint reverse sweep");
   }
   // Sub-windows of m steps (the whole window when the context's sub-window length is 0 or
@@ -1164,10 +1164,10 @@ int awfl_step_adjoint(awfl_ctx *c, const void *d_state_ckpt, void *d_lambda, int
       A.ca.dt = dt;
       A.ca.dens_c = c->d_dens_c; A.ca.denstheta_c = c->d_denstheta_c;
       A.ca.dens_g = c->d_dens_g; A.ca.denstheta_g = c->d_denstheta_g; A.ca.pres_g = c->d_pres_g;
-      e = launch_adjoint_split(ord, dir, A, 0, c->nsm, st);
+      e = launch_adjoint_split(ord, dir, A, 0, st);
     }
   }
-  if (e == cudaSuccess) e = launch_zero_halo((double *)d_lambda, nx, ny, nz, c->hs, c->nsm, st);
+  if (e == cudaSuccess) e = launch_zero_halo((double *)d_lambda, nx, ny, nz, c->hs, st);
   if (e != cudaSuccess) return cuda_fail(c, e, "adjoint reverse sweep");
   return AWFL_OK;
 }

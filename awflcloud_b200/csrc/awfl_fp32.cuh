@@ -471,8 +471,10 @@ struct P32 {
   // ord 5: five CTAs of 128 threads per SM (86-93 registers): 256x256x128 step 1.160 ms,
   // against 1.200 at the compiler's 115 (four) and 1.177 at six (80); the small-grid shapes
   // and the x-slab sweep at four (awfl_sweep.cuh)
-  // ord 9: three (168 registers, no spills by cp.async): 128x128x64 step 0.476 ms at two CTAs,
-  // 0.433 at three
+  // ord 9: three (168 registers by cp.async: the large grids' shapes spill nothing, the small
+  // ones' and the x-slab sweep 24-52 bytes): 128x128x64 step 0.476 ms at two CTAs, 0.433 at
+  // three. The ensembles' TMA kernels take the same bound for 128-thread tiles (40-60 bytes of
+  // spills, 230 registers at 64 threads; awfl_ensemble_tune picks)
   static constexpr int min_blocks(int ord) { return ord == 5 ? 5 : 3; }
   using Args = SweepArgs32;
   // where the base shape's rows come by TMA (`tma`), those that it cannot address (16-byte

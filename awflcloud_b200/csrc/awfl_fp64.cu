@@ -29,9 +29,10 @@ SweepChoice sweep_choice_fp64(int ord, int dir, const SweepArgs &A) { return swe
 
 // ------------------------------------------------------------------------------------
 // K6 apply (Temporal_ader.h:63-65): state(l,hs+k,hs+j,hs+i) += dt * tend(l,k,j,i). A thread
-// takes one cell's five variables: one index division per cell, ten loads in flight. Bound by
-// its bytes (120 per cell); 256x256x128: 308 -> 171 us, 0.91 of the
-// measured copy bandwidth; 130x100x70: 31.5 -> 14.7.
+// takes one cell's five variables: one index division per cell (a variable's store keeps the
+// next one's loads behind it, so two are in flight per thread). Bound by its bytes (120 per
+// cell); 256x256x128: 308 -> 171 us, 0.91 of the measured copy bandwidth; 130x100x70: 31.5 ->
+// 14.7.
 // ------------------------------------------------------------------------------------
 constexpr int kCellThreads = 256;
 // threads over the cells of a plane (x), planes (y)
@@ -60,8 +61,7 @@ __global__ void __launch_bounds__(kCellThreads) apply_kernel(double *state, cons
 }
 
 cudaError_t launch_apply_fp64(double *state, const double *tend, double dt, int nx, int ny, int nz, int hs,
-                              int nsm, cudaStream_t st) {
-  (void)nsm;
+                              cudaStream_t st) {
   apply_kernel<<<cell_grid(nx, ny, nz), kCellThreads, 0, st>>>(state, tend, dt, nx, ny, nz, hs);
   return cudaGetLastError();
 }
@@ -81,8 +81,7 @@ __global__ void __launch_bounds__(kCellThreads) apply32_kernel(float *state, flo
 }
 
 cudaError_t launch_apply_fp32(float *state, float *comp, const float *tend, float dt, int nx, int ny, int nz, int hs,
-                              int nsm, cudaStream_t st) {
-  (void)nsm;
+                              cudaStream_t st) {
   apply32_kernel<<<cell_grid(nx, ny, nz), kCellThreads, 0, st>>>(state, comp, tend, dt, nx, ny, nz, hs);
   return cudaGetLastError();
 }
@@ -97,8 +96,7 @@ __global__ void __launch_bounds__(kCellThreads) add_zero_kernel(double *x, int n
   for (int l = 0; l < nplanes; l++) x[p.s + l * sv] = __dadd_rn(x[p.s + l * sv], 0.0);
 }
 
-cudaError_t launch_add_zero_fp64(double *p, int nplanes, int nx, int ny, int nz, int hs, int nsm, cudaStream_t st) {
-  (void)nsm;
+cudaError_t launch_add_zero_fp64(double *p, int nplanes, int nx, int ny, int nz, int hs, cudaStream_t st) {
   add_zero_kernel<<<cell_grid(nx, ny, nz), kCellThreads, 0, st>>>(p, nplanes, nx, ny, nz, hs);
   return cudaGetLastError();
 }

@@ -165,7 +165,7 @@ SweepChoice sweep_choice_fp64(int ord, int dir, const SweepArgs &A);
 SweepChoice sweep_choice_tracers(int ord, int dir, const SweepArgs &A);
 SweepChoice sweep_choice_rec(int ord, int dir, const SweepArgs &A);
 cudaError_t launch_apply_fp32(float *state, float *comp, const float *tend, float dt, int nx, int ny, int nz, int hs,
-                              int nsm, cudaStream_t st);
+                              cudaStream_t st);
 cudaError_t upload_tables_fp32(int ord, const double *recon, const double *c2g, const double *s2g,
                                const double *deriv, const double *idl, double sigma, const double *wts);
 
@@ -219,13 +219,13 @@ cudaError_t launch_split_tracers32(int ord, int dir, const SweepArgs32 &A, const
 cudaError_t upload_tables_tracers32(int ord, const double *recon, const double *c2g, const double *s2g,
                                     const double *deriv, const double *idl, double sigma, const double *wts);
 // Adjoint reverse sweeps (awfl_adjrev.cu)
-cudaError_t launch_adjoint_split(int ord, int dir, const adj::SplitArgs &A, int need_edges, int nsm, cudaStream_t st);
-cudaError_t launch_zero_halo(double *lam, int nx, int ny, int nz, int hs, int nsm, cudaStream_t st);
+cudaError_t launch_adjoint_split(int ord, int dir, const adj::SplitArgs &A, int need_edges, cudaStream_t st);
+cudaError_t launch_zero_halo(double *lam, int nx, int ny, int nz, int hs, cudaStream_t st);
 cudaError_t upload_tables_adjrev(int ord, const void *tab, size_t bytes);
 cudaError_t launch_apply_fp64(double *state, const double *tend, double dt, int nx, int ny, int nz, int hs,
-                              int nsm, cudaStream_t st);
+                              cudaStream_t st);
 // x += dt*0 on the interior of nplanes planes (the sim2d y split's apply of zero tendencies)
-cudaError_t launch_add_zero_fp64(double *p, int nplanes, int nx, int ny, int nz, int hs, int nsm, cudaStream_t st);
+cudaError_t launch_add_zero_fp64(double *p, int nplanes, int nx, int ny, int nz, int hs, cudaStream_t st);
 // The largest max|u +- cs|, |v +- cs|, |w +- cs| of a state into result[0..2]; acc: four
 // device words, zero before the first call and after each.
 cudaError_t launch_cfl(const void *state, int fp32, const double *dens_c, const double *denstheta_c, int nx, int ny,

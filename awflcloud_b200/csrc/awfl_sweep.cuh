@@ -743,9 +743,9 @@ cudaError_t launch_sweep_shape(const typename P::Args &A, cudaStream_t st) {
     // 8 x 16: 148 168 155 us, by cp.async 138 158 140)
     typename P::Args a = A;
     if (P::prepare_tma(a, ORD, DIR, C, W)) {
-      if constexpr (DIR == 0 && P::kSlab && base)
+      if constexpr (DIR == 0 && P::kSlab)
         if (slab) return launch_sweep_kernel<P, ORD, DIR, C, W, true, true, false>(a, grid, st);
-      return launch_sweep_kernel<P, ORD, DIR, C, W, true, false, !base>(a, grid, st);
+      return launch_sweep_kernel<P, ORD, DIR, C, W, true, false, false>(a, grid, st);
     }
   }
   if constexpr (DIR == 0 && P::kSlab && base)
@@ -810,7 +810,7 @@ cudaError_t launch_sweep_t(const typename P::Args &A, cudaStream_t st) {
   using S = PolicyShapes<P, ORD, DIR>;
   if constexpr (S::n > 0) {
     const int best = sweep_shape<P, ORD, DIR>(A);
-    if constexpr (S::n > 0) if (best == 0) return launch_sweep_shape<P, ORD, DIR, S::C[0], S::W[0]>(A, st);
+    if (best == 0) return launch_sweep_shape<P, ORD, DIR, S::C[0], S::W[0]>(A, st);
     if constexpr (S::n > 1) if (best == 1) return launch_sweep_shape<P, ORD, DIR, S::C[1], S::W[1]>(A, st);
     if constexpr (S::n > 2) if (best == 2) return launch_sweep_shape<P, ORD, DIR, S::C[2], S::W[2]>(A, st);
     if constexpr (S::n > 3) if (best == 3) return launch_sweep_shape<P, ORD, DIR, S::C[3], S::W[3]>(A, st);
