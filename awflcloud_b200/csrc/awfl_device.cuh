@@ -154,7 +154,10 @@ __device__ __forceinline__ void reconstruct_gll(const Sc (&sten)[ORD], Sc (&out)
 //   - the weights' divisions by div_near, interleaved (no branch per division), the bridge
 //     polynomial's by div_known; the mapping's constants come from the tables.
 // A stencil whose smoothness indicators leave the range in which these hold (tv^2 >= 2^300,
-// infinities and NaN among them) is left to the general routine: these return false.
+// infinities and NaN among them) is left to the general routine: these return false. Where all
+// values of a stencil are below about 1e-303 the shared products round as subnormal numbers:
+// the two then differ by up to 4 of the smallest one (5e-324), like quotients there
+// (awfl_div.cuh). Sending such stencils to the general routine cost the FP64 step with tracers 1.5%.
 // 256x256x128: ord 5 6.68 -> 4.86 ms per step; 128x128x64, ord 9: 3.99 -> 3.30 ms.
 template <int ORD>
 __device__ __forceinline__ bool weno_weights(const double (&tv)[(ORD + 3) / 2], double (&w)[(ORD + 3) / 2]) {
