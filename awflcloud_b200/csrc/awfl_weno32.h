@@ -9,9 +9,9 @@ namespace awfl {
 // The ord-5 WENO reconstruction to the three GLL points in differences of the stencil: with
 // d_i = u[i+1]-u[i] and s_i = d[i+1]-d[i], the three parabolas are u[2] - s_i/24 + a_i x +
 // (s_i/2) x^2 and the bridge polynomial has the few coefficients of w5, where the matrix
-// form multiplies 49 entries. Equal in exact arithmetic; about 100 FP32 instructions instead of 150, and u[2] enters the values unrounded.
-// The sweep is issue-bound: with the time series on point pairs
-// (Pts below), 1,500 -> 1,130 instructions per cell and split, 256x256x128 step 1.433 -> 1.200 ms.
+// form multiplies 49 entries. Equal in exact arithmetic; about 100 FP32 instructions instead of
+// 150, and u[2] enters the values unrounded. The sweep is issue-bound: with the time series on
+// point pairs (Pts, awfl_fp32.cuh), 1,500 -> 1,130 instructions per cell and split, 256x256x128 step 1.433 -> 1.200 ms.
 template <class T> __device__ __forceinline__ void weno_gll5(const T (&u)[5], T (&out)[3]) {
   using namespace w5;
   const T d0 = u[1] - u[0], d1 = u[2] - u[1], d2 = u[3] - u[2], d3 = u[4] - u[3];
